@@ -123,6 +123,8 @@ struct bfx_sim {
     double* mm_result = nullptr;
     int mm_blocks = 0;
     float* scratch_f32 = nullptr;  // canonical read-out staging (lazily)
+    FaceEquilibria faces{};        // far-field / velocity face values of the fused kernel,
+    bool inline_faces = false;     // which takes the faces itself (bulk_inline_faces)
     bool face_ready = false;       // the staged kernel takes the x faces' values (face_dev) without their fill
     float face_dev[2 * 19] = {};   // those values (stored deviations, host copy)
     bfx_run_sample* dsamples = nullptr;
@@ -227,6 +229,8 @@ FluidBuffers fluid_buffers(bfx_sim* s, uint8_t* mask) {
     b.tmap = s->tma_ok ? &s->tmap : nullptr;
     b.sm_count = s->sm_count;
     b.face_dev = s->face_ready ? s->face_dev : nullptr;
+    b.faces = s->inline_faces ? &s->faces : nullptr;
+    b.count_step = 0;
     return b;
 }
 
@@ -332,7 +336,23 @@ bool x_faces_constant(const bfx_config& c) { return faces_constant(c, 0, 1); }
 // interior neighbour, and a link whose solid source is a periodic image writes
 // a halo slot: those keep the fill first on the main stream.
 bool halo_beside_links(const bfx_sim* s) {
-    return s->moving() && s->side != nullptr && faces_constant(s->cfg);
+    return s->moving() && s->side != nullptr && faces_constant(s->cfg) && !s->inline_faces;
+}
+// Without geometry and without a body update the end of a step is its counter
+// alone: the fused kernel counts it (not BF16, whose stochastic stores read
+// the counter).
+bool step_counted_by_bulk(const bfx_sim* s) {
+    return !s->geometry() && !(s->cfg.free_flight && s->has_bird) && s->cfg.storage != BFX_STORAGE_BF16_DEVIATION;
+}
+
+// The halo fill the step's fused kernel needs, on one stream: none where it
+// takes the faces itself, the y / z faces for the staged kernel with x-face
+// values, or every face.
+void encode_halo(bfx_sim* s, const FluidBuffers& fb, bool yz_only, cudaStream_t st) {
+    if (s->inline_faces) return;
+    if (yz_only) launch_halo_yz(s->cfg.storage, s->rep_s, s->g, s->fp, fb, st);
+    else launch_halo(s->cfg.storage, s->rep_s, s->g, s->fp, fb, st);
+    s->launches += 1;
 }
 
 // The cut-link and topology-event lists of a step's geometry, on the
@@ -404,10 +424,8 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     if (halo_side) {
         cudaEventRecord(s->halo_fork_ev, s->stream);
         cudaStreamWaitEvent(s->side, s->halo_fork_ev, 0);
-        if (yz_only) launch_halo_yz(s->cfg.storage, s->rep_s, s->g, s->fp, fb, s->side);
-        else launch_halo(s->cfg.storage, s->rep_s, s->g, s->fp, fb, s->side);
+        encode_halo(s, fb, yz_only, s->side);
         cudaEventRecord(s->halo_join_ev, s->side);
-        s->launches += 1;
     }
     if (s->moving() && !geometry_ready) {
         encode_geometry_build(s, 0, mprev, mnext);
@@ -443,17 +461,15 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     }
     // halo fill before the link writes: a link whose solid source is a periodic
     // image writes into a halo slot and must win over the periodic copy
-    if (!halo_side) {
-        if (yz_only) launch_halo_yz(s->cfg.storage, s->rep_s, s->g, s->fp, fb, s->stream);
-        else launch_halo(s->cfg.storage, s->rep_s, s->g, s->fp, fb, s->stream);
-        s->launches += 1;
-    }
+    if (!halo_side) encode_halo(s, fb, yz_only, s->stream);
     // The end-of-step body update needs only the reduced loads: it runs in the
     // link kernel's last block, except while taping (the tape records the
     // state between the loads and the body update).
     const FinishParams fin = {{s->cfg.gravity[0], s->cfg.gravity[1], s->cfg.gravity[2]}, (int)s->cfg.body_substeps,
                               s->cfg.free_flight && s->has_bird ? 1 : 0};
     const bool finish_fused = s->geometry() && !tape;
+    const bool counted = step_counted_by_bulk(s);
+    fb.count_step = counted ? 1 : 0;
     if (s->geometry()) {
         GeomBuffers gb = geom_buffers(s, mprev, mnext);
         if (tape) {
@@ -501,7 +517,7 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     }
     s->launches += launch_bulk_count(s->cfg.storage, s->cfg.collision, capture, s->tma_ok, s->geometry());
     GeomBuffers gb = geom_buffers(s, mprev, mnext);
-    if (!finish_fused) {
+    if (!finish_fused && !counted) {
         launch_integrate(s->g, s->fp, gb, fin.gravity[0], fin.gravity[1], fin.gravity[2], fin.substeps,
                          fin.free_flight, s->stream);
         s->launches += 1;
@@ -846,6 +862,9 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
     fp.act_margin = c.geometry == BFX_GEOMETRY_MESH
                         ? (int)std::ceil(c.mesh_half_thickness / c.cell_size) + 2 + 3
                         : 0;
+
+    s->inline_faces = bulk_inline_faces(c.storage, g, fp, c.geometry != BFX_GEOMETRY_NONE);
+    if (s->inline_faces) s->faces = make_face_equilibria(fp);
 
     s->elem = storage_bytes(c.storage);
     size_t pop_bytes = (size_t)19 * (size_t)g.padded * s->elem;

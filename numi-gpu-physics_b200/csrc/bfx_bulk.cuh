@@ -25,6 +25,9 @@ struct BulkArgs {
     // a population
     int face_values;
     float face_dev[2][19];
+    int inline_faces;       // k_bulk takes the faces itself (load_cell_edge), no halo fill
+    int count_step;         // the fused kernel also counts the step (no end-of-step kernel)
+    FaceEquilibria faces;
     int box[3];             // geometry box extent (origin in DeviceState); rare-cell launch
     void* pops;
     const uint8_t* mask;

@@ -258,6 +258,51 @@ __device__ __forceinline__ void load_cell(const BulkArgs& a, uint32_t pid, typen
     }
 }
 
+// load_cell of a warp that holds a boundary cell, without a halo fill (FP32 and
+// FP64).  A source beyond a periodic face is read at its image: f*_q(w) lies
+// in the slot A[opp q][w] (rep E) or A[q][w + c_q] (rep S), the normal slot
+// shifted by the axis' extent.  No cell of the step writes those slots (their
+// owner w + c_q lies outside the lattice), so the read needs no copy.  A source
+// beyond a far-field or velocity face takes the face's constant; one outside in
+// several open axes takes the x face first, then y, then z (exit_face).
+// Three passes without branches between the loads (address shifts, loads,
+// constants), so the 19 loads stay in flight together: with the rules decided at
+// each load the boundary warps ran one load latency after another.
+template <class S, int REP_S>
+__device__ __forceinline__ void load_cell_edge(const BulkArgs& a, int x, int y, int z, uint32_t pid,
+                                               typename S::R (&f)[19]) {
+    using T = typename S::T;
+    using R = typename S::R;
+    const Grid& g = a.g;
+    // beyond the low / high face of each axis: open, or periodic with its shift
+    const bool x0 = x == 0, x1 = x == g.nx - 1, y0 = y == 0, y1 = y == g.ny - 1, z0 = z == 0, z1 = z == g.nz - 1;
+    const bool ox0 = x0 && !g.per_x, ox1 = x1 && !g.per_x, oy0 = y0 && !g.per_y, oy1 = y1 && !g.per_y,
+               oz0 = z0 && !g.per_z, oz1 = z1 && !g.per_z;
+    const uint32_t ex = g.per_x ? (uint32_t)g.nx : 0u, ey = g.per_y ? (uint32_t)g.ny * (uint32_t)g.px : 0u,
+                   ez = g.per_z ? (uint32_t)g.nz * (uint32_t)g.pxy : 0u;
+    const uint32_t sx0 = x0 ? ex : 0u, sx1 = x1 ? 0u - ex : 0u, sy0 = y0 ? ey : 0u, sy1 = y1 ? 0u - ey : 0u,
+                   sz0 = z0 ? ez : 0u, sz1 = z1 ? 0u - ez : 0u;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) {
+        // with an open axis too the load only has to stay in the plane: the constant replaces it
+        const uint32_t shift = (cx(q) > 0 ? sx0 : (cx(q) < 0 ? sx1 : 0u)) + (cy(q) > 0 ? sy0 : (cy(q) < 0 ? sy1 : 0u)) +
+                               (cz(q) > 0 ? sz0 : (cz(q) < 0 ? sz1 : 0u));
+        if (REP_S) f[q] = S::ld_rt((const T*)a.plane[q] + (uint32_t)(pid + shift), q);
+        else f[q] = S::ld_rt((const T*)a.plane[opp(q)] + (uint32_t)(pid - (uint32_t)a.doff[q] + shift), opp(q));
+    }
+    // constants of the open faces, z first so that the x face wins
+    const auto face = [&](int k, int q) { return sizeof(R) == 8 ? (R)a.faces.d[k][q] : (R)a.faces.f[k][q]; };
+#pragma unroll
+    for (int k = 5; k >= 0; --k) {
+        const bool out = k == 0 ? ox0 : (k == 1 ? ox1 : (k == 2 ? oy0 : (k == 3 ? oy1 : (k == 4 ? oz0 : oz1))));
+#pragma unroll
+        for (int q = 1; q < 19; ++q) {
+            const int c = k < 2 ? cx(q) : (k < 4 ? cy(q) : cz(q));
+            if (c == ((k & 1) ? -1 : 1)) f[q] = out ? face(k, q) : f[q];
+        }
+    }
+}
+
 template <class S, int REP_S>
 __device__ __forceinline__ void store_cell(const BulkArgs& a, uint32_t pid, const typename S::R (&post)[19]) {
     using T = typename S::T;
@@ -392,9 +437,12 @@ __device__ __forceinline__ void rare_cell(const BulkArgs& a, uint32_t gid, int x
 
 // ---------------------------------------------------------------------------
 // The fused kernel: every cell of the lattice; solid and newly uncovered
-// cells (flagged in the mask) take rare_cell.
+// cells (flagged in the mask) take rare_cell.  FACES 1 (FP32 and FP64 on small
+// lattices, bulk_inline_faces) also takes the lattice faces, so no halo fill
+// precedes the kernel: its launch was a third of the step on a 64^3 periodic
+// lattice.
 // ---------------------------------------------------------------------------
-template <class S, int REP_S, int COLL, int CAPTURE>
+template <class S, int REP_S, int COLL, int CAPTURE, int FACES>
 __global__ void __launch_bounds__(256, sizeof(typename S::R) == 8 ? 1 : (COLL == BFX_COLLISION_TRT_LIMITER ? 2 : 4))
     k_bulk(const BulkArgs a) {
     using R = typename S::R;
@@ -405,6 +453,8 @@ __global__ void __launch_bounds__(256, sizeof(typename S::R) == 8 ? 1 : (COLL ==
     const uint32_t gid = (uint32_t)x + (uint32_t)a.g.nx * ((uint32_t)y + (uint32_t)a.g.ny * (uint32_t)z);
     const uint32_t pid =
         (uint32_t)(x + 1) + (uint32_t)a.g.px * ((uint32_t)(y + 1) + (uint32_t)a.g.py * (uint32_t)(z + 1));
+    // the step counter's only readers are the stochastic stores
+    if (!S::kStochastic && gid == 0 && a.count_step) a.state->step += 1;
     if (a.mask) {
         const uint8_t m = a.mask[gid];
         if (m) {
@@ -413,7 +463,13 @@ __global__ void __launch_bounds__(256, sizeof(typename S::R) == 8 ? 1 : (COLL ==
         }
     }
     R f[19];
-    load_cell<S, REP_S>(a, pid, f);
+    if constexpr (FACES) {
+        const bool edge = x == 0 || x == a.g.nx - 1 || y == 0 || y == a.g.ny - 1 || z == 0 || z == a.g.nz - 1;
+        if (__any_sync(__activemask(), edge)) load_cell_edge<S, REP_S>(a, x, y, z, pid, f);
+        else load_cell<S, REP_S>(a, pid, f);
+    } else {
+        load_cell<S, REP_S>(a, pid, f);
+    }
     R post[19];
     float activation = 0.0f, restriction = 0.0f;
     if constexpr (COLL == BFX_COLLISION_RR3 || COLL == BFX_COLLISION_REGULARIZED) {
@@ -501,11 +557,23 @@ template <class S, int REP, int COLL>
 static void bulk_t(const BulkArgs& a, const GridDesc& g, cudaStream_t s) {
     dim3 grid, block;
     cell_launch_shape(g, grid, block);
-    if (a.capture == 1) k_bulk<S, REP, COLL, 1><<<grid, block, 0, s>>>(a);
+    if constexpr (sizeof(typename S::T) >= 4) {
+        if (a.inline_faces) {
+            if (a.capture == 1) k_bulk<S, REP, COLL, 1, 1><<<grid, block, 0, s>>>(a);
 #ifndef BFX_CONTRACTED
-    else if (a.capture == 2 && COLL == BFX_COLLISION_TRT) k_bulk<S, REP, BFX_COLLISION_TRT, 2><<<grid, block, 0, s>>>(a);
+            else if (a.capture == 2 && COLL == BFX_COLLISION_TRT)
+                k_bulk<S, REP, BFX_COLLISION_TRT, 2, 1><<<grid, block, 0, s>>>(a);
 #endif
-    else k_bulk<S, REP, COLL, 0><<<grid, block, 0, s>>>(a);
+            else k_bulk<S, REP, COLL, 0, 1><<<grid, block, 0, s>>>(a);
+            return;
+        }
+    }
+    if (a.capture == 1) k_bulk<S, REP, COLL, 1, 0><<<grid, block, 0, s>>>(a);
+#ifndef BFX_CONTRACTED
+    else if (a.capture == 2 && COLL == BFX_COLLISION_TRT)
+        k_bulk<S, REP, BFX_COLLISION_TRT, 2, 0><<<grid, block, 0, s>>>(a);
+#endif
+    else k_bulk<S, REP, COLL, 0, 0><<<grid, block, 0, s>>>(a);
 }
 
 template <class S>

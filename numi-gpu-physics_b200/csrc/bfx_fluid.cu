@@ -16,8 +16,6 @@
 
 namespace bfx {
 
-
-
 // ---------------------------------------------------------------------------
 // Halo fill.  For every halo cell h and direction q whose target h + c_q is a
 // real cell b, write the population b pulls from outside the lattice into the
@@ -272,6 +270,26 @@ static size_t elem_bytes(int storage) {
     return storage == BFX_STORAGE_F64 ? 8 : (storage == BFX_STORAGE_F32 ? 4 : 2);
 }
 
+FaceEquilibria make_face_equilibria(const FluidParams& fp) {
+    FaceEquilibria e;
+    for (int f = 0; f < 6; ++f) {
+        const bool velocity = fp.face_bc[f] == BFX_BC_VELOCITY;
+        const float* u = velocity ? fp.face_u[f] : fp.far;
+        for (int q = 0; q < 19; ++q) {
+            e.f[f][q] = host_feq<float>(q, fp.far[3], u[0], u[1], u[2]);
+            e.d[f][q] = host_feq<double>(q, (double)fp.far[3], (double)u[0], (double)u[1], (double)u[2]);
+        }
+    }
+    return e;
+}
+
+bool bulk_inline_faces(int storage, const GridDesc& g, const FluidParams& fp, bool geometry) {
+    if (storage != BFX_STORAGE_F32 && storage != BFX_STORAGE_F64) return false;
+    for (int f = 0; f < 6; ++f)
+        if (fp.face_bc[f] == BFX_BC_OUTFLOW || (fp.face_bc[f] == BFX_BC_PERIODIC && geometry)) return false;
+    return g.n <= kInlineFaceCells;
+}
+
 Grid device_grid(const GridDesc& gd) {
     Grid g;
     g.nx = gd.nx;
@@ -306,6 +324,9 @@ BulkArgs make_bulk_args(const GridDesc& gd, const FluidParams& fp, const FluidBu
     a.face_values = b.face_dev ? 1 : 0;
     for (int f = 0; f < 2; ++f)
         for (int q = 0; q < 19; ++q) a.face_dev[f][q] = b.face_dev ? b.face_dev[19 * f + q] : 0.0f;
+    if (b.faces) a.faces = *b.faces;
+    a.inline_faces = b.faces ? 1 : 0;
+    a.count_step = b.count_step;
     a.pops = b.pops;
     a.mask = b.mask;
     a.wall = b.wall;

@@ -280,6 +280,8 @@ __global__ void __maxnreg__(StreamShape<COLL>::max_regs)
     }
     __syncthreads();
     const Grid& g = a.g;
+    // the step counter's only readers are the stochastic stores
+    if (!S::kStochastic && a.count_step && blockIdx.x == 0 && threadIdx.x == 0) a.state->step += 1;
     // bounded waits; the test hook can shorten them and withhold one tile
     const uint32_t hook_limit = a.state->test_wait_limit;
     const uint32_t wait_limit = hook_limit ? hook_limit : kWaitLimit;

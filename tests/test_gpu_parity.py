@@ -424,3 +424,44 @@ def test_prescribed_flapping_wing_matches_oracle_over_a_cycle():
     assert covered > 0
     assert len(cell) > 100
     lat.close()
+
+
+# --------------------------------------------------------------------------
+# Lattice faces taken by the FP32 / FP64 fused kernel (load_cell_edge), and the
+# combinations that keep the halo fill
+# --------------------------------------------------------------------------
+FF, PE, VE, OU = L.BC_FARFIELD, L.BC_PERIODIC, L.BC_VELOCITY, L.BC_OUTFLOW
+
+
+@pytest.mark.parametrize("faces", [[PE] * 6, [FF] * 6, [VE, FF, PE, PE, FF, VE], [PE, PE, VE, FF, PE, PE],
+                                   [VE, FF, VE, VE, FF, VE], [VE, OU, PE, PE, FF, VE], [OU, OU, VE, OU, OU, FF]])
+@pytest.mark.parametrize("extent", [(33, 10, 17), (64, 9, 8), (5, 4, 7)])
+@pytest.mark.parametrize("geometry", [False, True])
+def test_lattice_faces_match_oracle(faces, extent, geometry):
+    """Every kind of face, edge and corner bit for bit against the oracle; FP64 within FP32
+    rounding."""
+    nx, ny, nz = extent
+    cfg, rows, body, _ = cases.ellipsoid_channel(nx=nx, ny=ny, nz=nz, radii=(1.2, 1.1, 1.4),
+                                                 center=(0.5 * nx, 0.5 * ny, 0.5 * nz), viscosity=0.03,
+                                                 collision=L.COLLISION_TRT)
+    if not geometry:
+        cfg.geometry, rows, body = L.GEOMETRY_NONE, None, None
+    cfg.face_bc[:] = faces
+    for f in range(6):
+        cfg.face_velocity[f][:] = [0.04 - 0.01 * f, 0.01 * f, 0.005 * (f - 2)]
+    lat, osim = make_pair(cfg, rows, body)
+    rng = np.random.default_rng(3)
+    start = (lat.populations() * rng.uniform(0.97, 1.03, (19, nz, ny, nx))).astype(np.float32)
+    lat.set_populations(start)
+    osim.pa[:] = start.ravel()
+    for step in range(5):
+        lat.advance(1)
+        osim.step()
+        assert compare_pops(lat, osim, f"step {step + 1}")[1]
+    assert lat.step_index()[0] == 5
+    cfg.storage = L.STORAGE_F64
+    wide = Lattice(cfg, bird_struct(rows) if geometry else None, body_struct_from_tuple(body) if geometry else None)
+    wide.set_populations(start)
+    wide.advance(5)
+    # 5 steps of FP32 arithmetic: below 5 x 20 roundings of values near 1/3
+    assert np.max(np.abs(wide.populations() - lat.populations())) < 100 * 2.0 ** -25
