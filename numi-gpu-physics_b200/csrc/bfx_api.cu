@@ -125,8 +125,8 @@ struct bfx_sim {
     float* scratch_f32 = nullptr;  // canonical read-out staging (lazily)
     FaceEquilibria faces{};        // far-field / velocity face values of the fused kernel,
     bool inline_faces = false;     // which takes the faces itself (bulk_inline_faces)
-    bool face_ready = false;       // the staged kernel takes the x faces' values (face_dev) without their fill
-    float face_dev[2 * 19] = {};   // those values (stored deviations, host copy)
+    int face_ready = 0;            // faces the staged kernel takes from face_dev without their fill: 0, 2 (x) or 6
+    float face_dev[6 * 19] = {};   // their values (stored deviations, host copy)
     bfx_run_sample* dsamples = nullptr;
     size_t dsamples_cap = 0;
     // state
@@ -229,6 +229,7 @@ FluidBuffers fluid_buffers(bfx_sim* s, uint8_t* mask) {
     b.tmap = s->tma_ok ? &s->tmap : nullptr;
     b.sm_count = s->sm_count;
     b.face_dev = s->face_ready ? s->face_dev : nullptr;
+    b.face_count = s->face_ready;
     b.faces = s->inline_faces ? &s->faces : nullptr;
     b.count_step = 0;
     return b;
@@ -336,7 +337,7 @@ bool x_faces_constant(const bfx_config& c) { return faces_constant(c, 0, 1); }
 // interior neighbour, and a link whose solid source is a periodic image writes
 // a halo slot: those keep the fill first on the main stream.
 bool halo_beside_links(const bfx_sim* s) {
-    return s->moving() && s->side != nullptr && faces_constant(s->cfg) && !s->inline_faces;
+    return s->moving() && s->side != nullptr && faces_constant(s->cfg) && !s->inline_faces && s->face_ready != 6;
 }
 // Without geometry and without a body update the end of a step is its counter
 // alone: the fused kernel counts it (not BF16, whose stochastic stores read
@@ -348,8 +349,9 @@ bool step_counted_by_bulk(const bfx_sim* s) {
 // The halo fill the step's fused kernel needs, on one stream: none where it
 // takes the faces itself, the y / z faces for the staged kernel with x-face
 // values, or every face.
-void encode_halo(bfx_sim* s, const FluidBuffers& fb, bool yz_only, cudaStream_t st) {
-    if (s->inline_faces) return;
+void encode_halo(bfx_sim* s, const FluidBuffers& fb, bool staged, cudaStream_t st) {
+    const bool yz_only = staged && s->face_ready != 0;
+    if (s->inline_faces || (staged && s->face_ready == 6)) return;
     if (yz_only) launch_halo_yz(s->cfg.storage, s->rep_s, s->g, s->fp, fb, st);
     else launch_halo(s->cfg.storage, s->rep_s, s->g, s->fp, fb, st);
     s->launches += 1;
@@ -417,14 +419,13 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     uint8_t* mnext = s->moving() ? s->mask[s->cur ^ 1] : s->mask[s->cur];
     FluidBuffers fb = fluid_buffers(s, s->geometry() ? mnext : nullptr);
     // The halo fill forks off here (after the previous step's fluid kernel)
-    // and joins before this step's fluid kernel; without the x faces when
-    // the staged kernel takes their values from its table
-    const bool yz_only = s->face_ready && bulk_staged(s->cfg.storage, s->cfg.collision, tape ? 2 : capture, s->tma_ok);
+    // and joins before this step's fluid kernel
+    const bool staged = bulk_staged(s->cfg.storage, s->cfg.collision, tape ? 2 : capture, s->tma_ok);
     const bool halo_side = halo_beside_links(s) && !tape && !ledger_in;
     if (halo_side) {
         cudaEventRecord(s->halo_fork_ev, s->stream);
         cudaStreamWaitEvent(s->side, s->halo_fork_ev, 0);
-        encode_halo(s, fb, yz_only, s->side);
+        encode_halo(s, fb, staged, s->side);
         cudaEventRecord(s->halo_join_ev, s->side);
     }
     if (s->moving() && !geometry_ready) {
@@ -461,7 +462,7 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     }
     // halo fill before the link writes: a link whose solid source is a periodic
     // image writes into a halo slot and must win over the periodic copy
-    if (!halo_side) encode_halo(s, fb, yz_only, s->stream);
+    if (!halo_side) encode_halo(s, fb, staged, s->stream);
     // The end-of-step body update needs only the reduced loads: it runs in the
     // link kernel's last block, except while taping (the tape records the
     // state between the loads and the body update).
@@ -883,10 +884,9 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
                 staged_collision(c.collision) &&
                 encode_population_map(&s->tmap, s->pops, c.storage, c.collision, g.px, g.ny + 2, g.nz + 2);
     if (s->tma_ok) prepare_stream(c.storage, c.collision);
-    // Both x faces far-field or velocity faces: what the halo fill writes
-    // there depends on the face and the direction only, so the staged kernel
-    // takes it from a table and its steps skip the x faces' fill (one
-    // scattered store per lattice row and direction).
+    // Both x faces (or all six) far-field or velocity faces: what the halo fill
+    // writes there depends on the face and the direction only, so the staged
+    // kernel takes it from a table and its steps skip those faces' fill.
     if (s->tma_ok && x_faces_constant(c)) {
         float* dvals = nullptr;
         BFX_ALLOC(dvals, sizeof(s->face_dev));
@@ -898,7 +898,7 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
             bfx_destroy(s);
             return code;
         }
-        s->face_ready = true;
+        s->face_ready = faces_constant(c) ? 6 : 2;
     }
     BFX_ALLOC(s->density, (size_t)g.n * sizeof(float));
     BFX_ALLOC(s->velocity, (size_t)g.n * sizeof(float4));

@@ -96,17 +96,16 @@ __global__ void __launch_bounds__(128) k_halo(const BulkArgs a, int rep_s, int64
 }
 
 // The values k_halo writes across a far-field or velocity face depend only on
-// the face and the direction.  When both x faces are of those kinds the
-// staged kernel takes their values from this table instead of the x-halo
-// slots, whose fill (one scattered store per row and direction) it skips:
-// out[19 f + q] = the stored value of direction q across face f (0: -x,
-// 1: +x), read back as the staged kernel reads a population (scaled deviation).
+// the face and the direction.  When both x faces (or all six) are of those
+// kinds the staged kernel takes their values from this table and their halo
+// fill is skipped (an x face's is one scattered store per row and direction):
+// out[19 f + q] = the stored value of direction q across face f, read back as the staged kernel reads a population (scaled deviation).
 template <class S>
 __global__ void k_halo_values(const BulkArgs a, float* out) {
     using T = typename S::T;
     using R = typename S::R;
     const int t = threadIdx.x;
-    if (t >= 2 * 19) return;
+    if (t >= 6 * 19) return;
     const int f = t / 19, q = t % 19;
     const FluidParams& fp = a.fp;
     R val = sizeof(R) == 8 ? (R)a.far_eq_d[q] : (R)a.far_eq_f[q];
@@ -321,8 +320,8 @@ BulkArgs make_bulk_args(const GridDesc& gd, const FluidParams& fp, const FluidBu
         const double scale = storage == BFX_STORAGE_F16_DEVIATION ? (double)StoreF16Dev::kDevScale : 1.0;
         a.far_dev[q] = (float)((a.far_eq_d[q] - wq<double>(q)) * scale);
     }
-    a.face_values = b.face_dev ? 1 : 0;
-    for (int f = 0; f < 2; ++f)
+    a.face_values = b.face_dev ? (b.face_count == 6 ? 2 : 1) : 0;
+    for (int f = 0; f < 6; ++f)
         for (int q = 0; q < 19; ++q) a.face_dev[f][q] = b.face_dev ? b.face_dev[19 * f + q] : 0.0f;
     if (b.faces) a.faces = *b.faces;
     a.inline_faces = b.faces ? 1 : 0;

@@ -38,8 +38,9 @@ struct FluidBuffers {
     int sm_count;
     const FaceEquilibria* faces;  // host copy; null: the halo fill covers the faces
     int count_step;         // the fused kernel counts the step (no geometry, no body update)
-    const float* face_dev;  // host copy of the x-face values [2][19] for the staged kernel (null: the halo
-                            // fill covers the x faces)
+    const float* face_dev;  // host copy of the face values [6][19] for the staged kernel (null: the halo
+                            // fill covers every face)
+    int face_count;         // faces the staged kernel takes from face_dev: 2 (-x, +x) or 6
 };
 
 // Fused stream + collide of every cell: fluid cells collide, solid cells take
@@ -52,8 +53,8 @@ void launch_bulk(int storage, int collision, int rep_s, const GridDesc& g, const
 // The step runs the TMA-staged kernel (16-bit storage, staged operator, a
 // population tensor map, not taped).
 bool bulk_staged(int storage, int collision, int capture, bool tma_ok);
-// x-face values for the staged kernel when both x faces are far-field or
-// velocity faces (BulkArgs::face_dev): out[2 * 19], computed as the halo fill
+// Far-field / velocity face values for the staged kernel (BulkArgs::face_dev):
+// out[6 * 19], computed as the halo fill
 // computes and stores them, read back as stored deviations.
 void launch_halo_values(int storage, const GridDesc& g, const FluidParams& fp, float* out, cudaStream_t s);
 // Halo fill of the z and y faces only (the staged kernel takes the x faces'

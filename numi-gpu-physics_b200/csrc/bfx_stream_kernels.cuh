@@ -174,6 +174,18 @@ __device__ __forceinline__ void collide_dev2(const P2 (&d)[19], float s, float i
     }
 }
 
+// y and z faces without their halo fill (face_values 2): a warp's cells lie in
+// one row, so the tests are warp-uniform and cost an interior tile two
+// compares.  Applied before the x faces, z first: the fill takes the x face,
+// then y, then z for a source outside in several axes.
+template <int F>
+__device__ __forceinline__ void row_face_values(const BulkArgs& a, P2 (&dv)[19]) {
+    constexpr int sgn = (F & 1) ? -1 : 1;
+#pragma unroll
+    for (int q = 1; q < 19; ++q)
+        if ((F < 4 ? cy(q) : cz(q)) == sgn) dv[q] = pv(a.face_dev[F][q]);
+}
+
 // x faces without their halo fill (BulkArgs::face_values): at x = 0 (SGN +1)
 // every direction with c_x > 0 comes from beyond the -x face, at x = nx - 1
 // (SGN -1) every direction with c_x < 0 from beyond the +x face; the halo
@@ -393,6 +405,12 @@ __global__ void __maxnreg__(StreamShape<COLL>::max_regs)
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(empty0 + 8 * s);
+        if (a.face_values == 2 && (y == 0 || y + 1 >= g.ny || z == 0 || z + 1 == g.nz)) {
+            if (z == 0) row_face_values<4>(a, dv);
+            if (z + 1 == g.nz) row_face_values<5>(a, dv);
+            if (y == 0) row_face_values<2>(a, dv);
+            if (y + 1 == g.ny) row_face_values<3>(a, dv);
+        }
         if (a.face_values) {
             // no x-halo fill: the warp's cells at x = 0 or x = nx - 1 take the
             // x-face values (one warp-uniform test for the warp's 64 cells)
