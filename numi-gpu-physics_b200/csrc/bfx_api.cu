@@ -965,7 +965,7 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
         BFX_ALLOC(s->topo_partials, (size_t)s->topo_blocks * 8 * sizeof(double));
         cudaMemsetAsync(s->topo_partials, 0, (size_t)s->topo_blocks * 8 * sizeof(double), s->stream);
         s->apply_blocks = 4 * s->sm_count;
-        BFX_ALLOC(s->link_partials, (size_t)s->apply_blocks * 16 * sizeof(double));
+        BFX_ALLOC(s->link_partials, (size_t)s->apply_blocks * 8 * sizeof(double));
         uint64_t cap = c.link_capacity ? c.link_capacity
                                        : std::max<uint64_t>(1u << 18, std::min<uint64_t>((uint64_t)s->box.cells, 1u << 24));
         s->link_capacity = (uint32_t)cap;

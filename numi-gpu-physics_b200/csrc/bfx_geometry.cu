@@ -1402,13 +1402,31 @@ __global__ void __launch_bounds__(128) k_links_fraction_ray(const GeomArgs a) {
 // the incoming population, write it where the fluid step will read it, and
 // accumulate the momentum-exchange load in FP64.
 // ---------------------------------------------------------------------------
+// The step's reduced loads (lattice force and power sums, physical torque).
+struct StepLoads {
+    double lattice[3], torque[3], power;
+};
 __device__ void finish_state(const GeomArgs& a, float gx, float gy, float gz, int substeps, int free_flight,
-                             const bfx_bird* bird_ptr);
+                             const bfx_bird* bird_ptr, const StepLoads& loads);
+
+// Sum of eight values over the lanes of a warp, in every lane (fixed order).
+__device__ __forceinline__ void warp_sum(double (&v)[8]) {
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+}
+
+// Bound by latency: a few ten thousand links are one per thread.  So only the
+// blocks that hold links take part (with every block of the fixed grid writing
+// and the last one reducing a row of partials, and FP64 shared-memory trees for
+// the sums, the kernel took 17 us on the coupled bird and 16 on the 256 x 128 x 128 channel), the sums run on shuffles, the last
+// block reads the topology partials itself and hands the loads to the body
+// update in registers: 10 and 9 us.
 
 template <class S>
 __global__ void __launch_bounds__(256) k_links_apply(const GeomArgs a, int rep_s, int with_topology, int fuse_finish,
                                                      const FinishParams fin) {
-    __shared__ double sh[8][256];
+    __shared__ double warp_sums[16][8];
     __shared__ int last_block;
     using T = typename S::T;
     using R = typename S::R;
@@ -1422,6 +1440,11 @@ __global__ void __launch_bounds__(256) k_links_apply(const GeomArgs a, int rep_s
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int64_t count = a.b.state->link_count;
     if (count > (int64_t)a.b.link_capacity) count = a.b.link_capacity;
+    // the blocks that hold links (at least one); the others leave at once
+    const int active = count > (int64_t)gridDim.x * blockDim.x ? (int)gridDim.x
+                       : count > 0                             ? (int)((count + blockDim.x - 1) / blockDim.x)
+                                                               : 1;
+    if ((int)blockIdx.x >= active) return;
     const R cs2 = Lat<R>::cs2;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t gid = a.b.link_cell[i];
@@ -1558,58 +1581,68 @@ __global__ void __launch_bounds__(256) k_links_apply(const GeomArgs a, int rep_s
             }
         }
     }
-    // Block sums: the link loads, then this block's contiguous share of the
-    // topology partials (most blocks hold no link and no topology impulse).
-    bool nonzero = false;
-    for (int k = 0; k < 8; ++k) nonzero = nonzero || acc[k] != 0.0;
-    if (__syncthreads_or(nonzero)) block_sum<8>(acc, sh);
-    double tp[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (with_topology) {
-        const int nb = a.b.topo_blocks;
-        const int per = (nb + (int)gridDim.x - 1) / (int)gridDim.x;
-        const int lo = (int)blockIdx.x * per;
-        const int hi = lo + per < nb ? lo + per : nb;
-        for (int i = lo + (int)threadIdx.x; i < hi; i += blockDim.x)
-            for (int k = 0; k < 8; ++k) tp[k] += a.b.topo_partials[8 * (int64_t)i + k];
-        bool tnz = false;
-        for (int k = 0; k < 8; ++k) tnz = tnz || tp[k] != 0.0;
-        if (__syncthreads_or(tnz)) block_sum<8>(tp, sh);
-    }
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < 8; ++k) {
-            a.b.link_partials[16 * blockIdx.x + k] = acc[k];
-            a.b.link_partials[16 * blockIdx.x + 8 + k] = tp[k];
-        }
+    // Block sums of the link loads: warp shuffles, then one thread per value
+    // over the warps (fixed order).
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    warp_sum(acc);
+    if (lane == 0)
+        for (int k = 0; k < 8; ++k) warp_sums[k][warp] = acc[k];
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        double v = 0.0;
+        for (int w = 0; w < 8; ++w) v += warp_sums[threadIdx.x][w];
+        a.b.link_partials[8 * blockIdx.x + threadIdx.x] = v;
         __threadfence();
-        last_block = atomicAdd(&a.b.state->apply_done, 1u) == gridDim.x - 1 ? 1 : 0;
     }
     __syncthreads();
+    if (threadIdx.x == 0)
+        last_block = atomicAdd(&a.b.state->apply_done, 1u) == (unsigned)active - 1u ? 1 : 0;
+    __syncthreads();
     if (!last_block) return;
-    // Last block: fixed-order sums of the per-block partials (the result does
-    // not depend on which block finishes last).
+    // Last block: fixed-order sums of the per-block link partials and of the
+    // topology partials (the result does not depend on which block finishes
+    // last).
     __threadfence();
     double l[8] = {0, 0, 0, 0, 0, 0, 0, 0}, t[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x)
+    for (int i = threadIdx.x; i < active; i += blockDim.x)
+        for (int k = 0; k < 8; ++k) l[k] += __ldcg(a.b.link_partials + 8 * i + k);
+    if (with_topology)
+        for (int i = threadIdx.x; i < a.b.topo_blocks; i += blockDim.x)
+            for (int k = 0; k < 8; ++k) t[k] += a.b.topo_partials[8 * i + k];
+    warp_sum(l);
+    if (with_topology) warp_sum(t);
+    if (lane == 0)
         for (int k = 0; k < 8; ++k) {
-            l[k] += __ldcg(a.b.link_partials + 16 * i + k);
-            t[k] += __ldcg(a.b.link_partials + 16 * i + 8 + k);
+            warp_sums[k][warp] = l[k];
+            warp_sums[8 + k][warp] = t[k];
         }
-    block_sum<8>(l, sh);
-    block_sum<8>(t, sh);
+    __syncthreads();
+    // each of the sixteen values over the warps, then handed to thread 0
+    if (threadIdx.x < 16) {
+        double v = 0.0;
+        for (int w = 0; w < 8; ++w) v += warp_sums[threadIdx.x][w];
+        warp_sums[threadIdx.x][0] = v;
+    }
+    __syncwarp();
     if (threadIdx.x == 0) {
         DeviceState* st = a.b.state;
+        StepLoads loads;
         for (int k = 0; k < 3; ++k) {
-            st->loads_lattice[k] = t[k] + l[k];
-            st->loads_torque[k] = t[3 + k] + l[3 + k];
+            loads.lattice[k] = warp_sums[8 + k][0] + warp_sums[k][0];
+            loads.torque[k] = warp_sums[11 + k][0] + warp_sums[3 + k][0];
+            st->loads_lattice[k] = loads.lattice[k];
+            st->loads_torque[k] = loads.torque[k];
         }
-        st->power_lattice = l[6];
+        loads.power = warp_sums[6][0];
+        st->power_lattice = loads.power;
         if (with_topology) {
-            st->covered_count = (int64_t)t[6];
-            st->uncovered_count = (int64_t)t[7];
+            st->covered_count = (int64_t)warp_sums[14][0];
+            st->uncovered_count = (int64_t)warp_sums[15][0];
         }
         st->apply_done = 0;
         if (fuse_finish)
-            finish_state(a, fin.gravity[0], fin.gravity[1], fin.gravity[2], fin.substeps, fin.free_flight, a.b.bird);
+            finish_state(a, fin.gravity[0], fin.gravity[1], fin.gravity[2], fin.substeps, fin.free_flight, a.b.bird,
+                         loads);
     }
 }
 
@@ -1630,16 +1663,16 @@ __device__ void qnormalize_d(double* q) {
 }
 
 __device__ void finish_state(const GeomArgs& a, float gx, float gy, float gz, int substeps, int free_flight,
-                             const bfx_bird* bird_ptr) {
+                             const bfx_bird* bird_ptr, const StepLoads& loads) {
     DeviceState* st = a.b.state;
     const FluidParams& fp = a.fp;
     if (free_flight) {
         const bfx_bird& bird = *bird_ptr;
         double force[3], torque[3];
         for (int k = 0; k < 3; ++k) {
-            force[k] = st->loads_lattice[k] * (double)fp.f2p;
+            force[k] = loads.lattice[k] * (double)fp.f2p;
             force[k] = force[k] + (double)st->wing_reaction[k] + (double)st->wing_reaction[8 + k];
-            torque[k] = st->loads_torque[k] + (double)st->wing_reaction[4 + k] + (double)st->wing_reaction[12 + k];
+            torque[k] = loads.torque[k] + (double)st->wing_reaction[4 + k] + (double)st->wing_reaction[12 + k];
         }
         int n = substeps < 1 ? 1 : substeps;
         double dt = (double)fp.dt / (double)n;
@@ -1731,8 +1764,8 @@ __device__ void finish_state(const GeomArgs& a, float gx, float gy, float gz, in
         if (k >= ob->first && k <= ob->last) {
             const double inv = 1.0 / (double)(ob->last - ob->first + 1);
             double j = 0.0;
-            for (int c = 0; c < 3; ++c) j += ob->force_weight[c] * (st->loads_lattice[c] * (double)fp.f2p);
-            j += ob->power_weight * (-st->power_lattice * (double)fp.f2p / (double)fp.v2l);
+            for (int c = 0; c < 3; ++c) j += ob->force_weight[c] * (loads.lattice[c] * (double)fp.f2p);
+            j += ob->power_weight * (-loads.power * (double)fp.f2p / (double)fp.v2l);
             ob->value += j * inv;
         }
     }
@@ -1741,7 +1774,14 @@ __device__ void finish_state(const GeomArgs& a, float gx, float gy, float gz, in
 
 __global__ void k_finish(const GeomArgs a, float gx, float gy, float gz, int substeps, int free_flight,
                          const bfx_bird* bird_ptr) {
-    finish_state(a, gx, gy, gz, substeps, free_flight, bird_ptr);
+    const DeviceState* st = a.b.state;
+    StepLoads loads;
+    for (int k = 0; k < 3; ++k) {
+        loads.lattice[k] = st->loads_lattice[k];
+        loads.torque[k] = st->loads_torque[k];
+    }
+    loads.power = st->power_lattice;
+    finish_state(a, gx, gy, gz, substeps, free_flight, bird_ptr, loads);
 }
 
 __global__ void k_record_sample(const GeomArgs a, bfx_run_sample* samples, uint64_t index, float dt) {

@@ -150,7 +150,7 @@ struct GeomBuffers {
     int scan_blocks;                // blocks of the link count / scan / emission launch
     double* topo_partials;          // 8 per topology block
     int topo_blocks;                // blocks of the topology-impulse launch
-    double* link_partials;          // 16 per apply block (link sums, topology sums)
+    double* link_partials;          // 8 per apply block
     int apply_blocks;
     DeviceState* state;
     Objective* objective;           // load objective accumulated by the step end (may be null)
