@@ -305,20 +305,19 @@ void encode_geometry_build(bfx_sim* s, int init, uint8_t* mprev, uint8_t* mnext,
     if (!st) st = s->stream;
     launch_prepare(s->cfg.geometry, s->cfg.time_step, s->g, s->fp, s->box, gb, init, st);
     // beside the TRT staged kernel (pipelined build): the register-lean raster
-    const bool lean = st == s->side && s->cfg.collision == BFX_COLLISION_TRT;
+    const bool lean = st == s->side && s->tma_ok && s->cfg.collision == BFX_COLLISION_TRT;
     launch_classify(s->cfg.geometry, init ? 0 : 1, s->g, s->fp, s->box, gb, st, lean);
     s->launches += 1 + (s->cfg.geometry == BFX_GEOMETRY_MESH ? 4 : 1);
 }
 
-// The next step's geometry build can overlap this step's fluid kernel: with
-// the staged 16-bit kernel the fluid cells read only the populations and this
-// step's mask, while the build writes the other mask buffer, the wall field,
-// the keys, the pose fields and link count of the device state, and the
-// cut-link and event lists (this step's link kernel has read them before the
-// fork); the body update it reads is done by the link kernel before the fluid
-// kernel, and the box's solid cells (which read the wall field) are launched
-// before the fork.
-bool can_pipeline(const bfx_sim* s) { return s->moving() && s->tma_ok && s->side != nullptr; }
+// The next step's geometry build can overlap this step's fluid kernel: the
+// fluid cells read only the populations and this step's mask, while the build
+// writes the other mask buffer, the wall field, the keys, the pose fields and
+// link count of the device state, and the cut-link and event lists (this
+// step's link kernel has read them before the fork); the body update it reads
+// is done by the link kernel before the fluid kernel, and the box's solid
+// cells (which read the wall field) are launched before the fork.
+bool can_pipeline(const bfx_sim* s) { return s->moving() && s->side != nullptr; }
 
 // Faces f0..f1 are far-field or velocity faces: the values the halo fill
 // writes there depend only on the face and the direction.
@@ -509,14 +508,14 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
         if (s->geometry()) encode_link_build(s, mnext, mprev, s->side, s->lists_ev);
         else cudaEventRecord(s->lists_ev, s->side);
         cudaEventRecord(s->join_ev, s->side);
-        launch_bulk_stream(s->cfg.storage, s->cfg.collision, s->rep_s, s->g, s->fp, fb, box, s->stream);
+        launch_bulk_fluid(s->cfg.storage, s->cfg.collision, s->rep_s, s->g, s->fp, fb, box, s->stream);
     } else {
         timing_begin(s);
         launch_bulk(s->cfg.storage, s->cfg.collision, s->rep_s, s->g, s->fp, fb, capture,
                     s->geometry() ? box : nullptr, s->stream);
         timing_end(s);
     }
-    s->launches += launch_bulk_count(s->cfg.storage, s->cfg.collision, capture, s->tma_ok, s->geometry());
+    s->launches += pipelined ? 2 : launch_bulk_count(s->cfg.storage, s->cfg.collision, capture, s->tma_ok, s->geometry());
     GeomBuffers gb = geom_buffers(s, mprev, mnext);
     if (!finish_fused && !counted) {
         launch_integrate(s->g, s->fp, gb, fin.gravity[0], fin.gravity[1], fin.gravity[2], fin.substeps,
@@ -787,23 +786,29 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
     s->device = config->device;
     cudaSetDevice(s->device);
     cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->device);
-    // The main stream (fluid kernel, link build) has the device's greatest
-    // priority and the side stream (the next step's geometry, the halo fill)
-    // its least: when both have blocks waiting, the persistent fluid kernel's
-    // CTAs are placed first and the side kernels fill the resources it leaves.
+    // Which of the two streams' waiting blocks is placed first.  The staged
+    // 16-bit kernel is persistent: its CTAs go first (main stream greatest,
+    // side stream least) and the side kernels fill the resources it leaves.
+    // k_bulk fills every SM block after block, so a side kernel of lesser
+    // priority would wait for its last wave: there the side stream (the next
+    // step's geometry, short and latency-bound) goes first.
     int least_priority = 0, greatest_priority = 0;
     if (cudaDeviceGetStreamPriorityRange(&least_priority, &greatest_priority) != cudaSuccess) {
         (void)cudaGetLastError();
         least_priority = greatest_priority = 0;
     }
-    cudaError_t e = cudaStreamCreateWithPriority(&s->stream, cudaStreamNonBlocking, greatest_priority);
+    const bool staged = (config->storage == BFX_STORAGE_F16_DEVIATION || config->storage == BFX_STORAGE_BF16_DEVIATION) &&
+                        staged_collision(config->collision);
+    const int main_priority = staged ? greatest_priority : least_priority;
+    const int side_priority = staged ? least_priority : greatest_priority;
+    cudaError_t e = cudaStreamCreateWithPriority(&s->stream, cudaStreamNonBlocking, main_priority);
     if (e != cudaSuccess) {
         bfx_destroy(s);
         return cuda_fail(nullptr, e, "stream creation");
     }
     // side stream for the pipelined geometry build (optional: without it the
     // steps run in order on the main stream)
-    if (cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, least_priority) != cudaSuccess ||
+    if (cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, side_priority) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->join_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->lists_ev, cudaEventDisableTiming) != cudaSuccess ||

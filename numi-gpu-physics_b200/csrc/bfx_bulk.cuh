@@ -26,6 +26,7 @@ struct BulkArgs {
     int face_values;
     float face_dev[6][19];
     int inline_faces;       // k_bulk takes the faces itself (load_cell_edge), no halo fill
+    int skip_rare;          // k_bulk leaves solid / newly uncovered cells to k_rare (pipelined step)
     int count_step;         // the fused kernel also counts the step (no end-of-step kernel)
     FaceEquilibria faces;
     int box[3];             // geometry box extent (origin in DeviceState); rare-cell launch

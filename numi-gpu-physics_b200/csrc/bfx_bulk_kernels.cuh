@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(256, sizeof(typename S::R) == 8 ? 1 : (COLL ==
     if (a.mask) {
         const uint8_t m = a.mask[gid];
         if (m) {
-            rare_cell<S, REP_S, COLL>(a, gid, x, y, z, pid, m);
+            if (!a.skip_rare) rare_cell<S, REP_S, COLL>(a, gid, x, y, z, pid, m);
             return;
         }
     }
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(256, sizeof(typename S::R) == 8 ? 1 : (COLL ==
 }
 
 // Solid / newly uncovered cells of the geometry box in a launch of their own
-// (the staged kernel skips them).  A thread scans kRareZ cells along z of one
+// (the staged kernel skips them, and k_bulk in a pipelined step).  A thread scans kRareZ cells along z of one
 // (x, y) column of the box, all mask bytes loaded before the first is used.
 constexpr int kRareZ = 8;
 template <class S, int REP_S, int COLL>

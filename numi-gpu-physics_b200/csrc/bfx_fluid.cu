@@ -326,6 +326,7 @@ BulkArgs make_bulk_args(const GridDesc& gd, const FluidParams& fp, const FluidBu
     if (b.faces) a.faces = *b.faces;
     a.inline_faces = b.faces ? 1 : 0;
     a.count_step = b.count_step;
+    a.skip_rare = 0;
     a.pops = b.pops;
     a.mask = b.mask;
     a.wall = b.wall;
@@ -414,6 +415,12 @@ int launch_bulk_count(int storage, int collision, int capture, bool tma_ok, bool
     return use_staged(storage, collision, capture, tma_ok) && geometry ? 2 : 1;
 }
 
+// The fused step of this storage runs the contracted translation unit.
+static bool contracted(int storage, const FluidParams& fp) {
+    return storage == BFX_STORAGE_F16_DEVIATION || storage == BFX_STORAGE_BF16_DEVIATION ||
+           (storage == BFX_STORAGE_F32 && fp.fast_math);
+}
+
 void launch_bulk(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
                  const FluidBuffers& b, int capture, const int* box, cudaStream_t s) {
     BulkArgs a = make_bulk_args(g, fp, b, capture, storage);
@@ -422,8 +429,6 @@ void launch_bulk(int storage, int collision, int rep_s, const GridDesc& g, const
         a.box[1] = box[1];
         a.box[2] = box[2];
     }
-    const bool contracted = storage == BFX_STORAGE_F16_DEVIATION || storage == BFX_STORAGE_BF16_DEVIATION ||
-                            (storage == BFX_STORAGE_F32 && fp.fast_math);
     // 16-bit TRT / regularized / RR3: the TMA-staged kernel, measured faster
     // there (16-bit loads leave k_bulk latency-bound; the packed pair
     // arithmetic halves the regularized operators' issue time), with the
@@ -435,7 +440,7 @@ void launch_bulk(int storage, int collision, int rep_s, const GridDesc& g, const
         if (box && a.mask) launch_rare_fast(storage, collision, rep_s, a, s);
         return;
     }
-    if (contracted) {
+    if (contracted(storage, fp)) {
         launch_bulk_fast(storage, collision, rep_s, g, a, s);
     } else if (storage == BFX_STORAGE_F64) {
         exact::bulk_s<StoreF64>(a, g, collision, rep_s, s);
@@ -444,22 +449,29 @@ void launch_bulk(int storage, int collision, int rep_s, const GridDesc& g, const
     }
 }
 
-// The staged path of launch_bulk in its two launches, so that other work can
+// launch_bulk of a pipelined step in its two launches, so that other work can
 // be queued between them: the geometry box's solid and newly uncovered cells
-// (k_rare), then the fluid cells (k_stream).  Every population slot is read
-// and written by one cell only in a step, and the two launches cover disjoint
-// cells, so their order does not change the result.
+// (k_rare), then the fluid cells.  Every population slot is read and written by
+// one cell only in a step, and the two launches cover disjoint cells, so their
+// order does not change the result.
 void launch_bulk_rare(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
                       const FluidBuffers& b, const int* box, cudaStream_t s) {
     BulkArgs a = make_bulk_args(g, fp, b, 0, storage);
     for (int k = 0; k < 3; ++k) a.box[k] = box[k];
-    launch_rare_fast(storage, collision, rep_s, a, s);
+    if (contracted(storage, fp)) launch_rare_fast(storage, collision, rep_s, a, s);
+    else if (storage == BFX_STORAGE_F64) exact::rare_s<StoreF64>(a, collision, rep_s, s);
+    else exact::rare_s<StoreF32>(a, collision, rep_s, s);
 }
-void launch_bulk_stream(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
-                        const FluidBuffers& b, const int* box, cudaStream_t s) {
+void launch_bulk_fluid(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
+                       const FluidBuffers& b, const int* box, cudaStream_t s) {
     BulkArgs a = make_bulk_args(g, fp, b, 0, storage);
     for (int k = 0; k < 3; ++k) a.box[k] = box[k];
-    launch_stream_fast(storage, collision, rep_s, g, &a, (const CUtensorMap*)b.tmap, b.sm_count, s);
+    a.skip_rare = 1;
+    if (use_staged(storage, collision, 0, b.tmap != nullptr))
+        launch_stream_fast(storage, collision, rep_s, g, &a, (const CUtensorMap*)b.tmap, b.sm_count, s);
+    else if (contracted(storage, fp)) launch_bulk_fast(storage, collision, rep_s, g, a, s);
+    else if (storage == BFX_STORAGE_F64) exact::bulk_s<StoreF64>(a, g, collision, rep_s, s);
+    else exact::bulk_s<StoreF32>(a, g, collision, rep_s, s);
 }
 
 template <class S>

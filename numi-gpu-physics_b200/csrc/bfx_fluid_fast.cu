@@ -17,7 +17,8 @@ void launch_stream_fast(int storage, int collision, int rep_s, const GridDesc& g
 
 void launch_rare_fast(int storage, int collision, int rep_s, const BulkArgs& a, cudaStream_t s) {
     if (storage == BFX_STORAGE_BF16_DEVIATION) fast::rare_s<StoreBF16Dev>(a, collision, rep_s, s);
-    else fast::rare_s<StoreF16Dev>(a, collision, rep_s, s);
+    else if (storage == BFX_STORAGE_F16_DEVIATION) fast::rare_s<StoreF16Dev>(a, collision, rep_s, s);
+    else fast::rare_s<StoreF32>(a, collision, rep_s, s);
 }
 
 void launch_bulk_fast(int storage, int collision, int rep_s, const GridDesc& g, const BulkArgs& a, cudaStream_t s) {

@@ -139,6 +139,7 @@ __global__ void k_prepare(const GeomArgs a, int init, float dt, float box_radius
         __syncthreads();
         if (t != 0) return;
     }
+    if (a.b.live_count) *a.b.live_count = 0;  // the resolve's list starts empty
     V3 pos = v3((float)sbody[0], (float)sbody[1], (float)sbody[2]);
     float4 orient = make_float4((float)sbody[3], (float)sbody[4], (float)sbody[5], (float)sbody[6]);
     V3 vel = v3((float)sbody[7], (float)sbody[8], (float)sbody[9]);
@@ -837,6 +838,8 @@ __device__ bool resolve_cell(const GeomArgs& a, int has_prev, int x, int y, int 
 // or a topology event, so the link count and emission visit those alone.  The
 // list's order is not fixed, and nothing depends on it: the counts are stored
 // by block index and the emission writes at offsets scanned in block order.
+// The other blocks' counts are zeroed here (by a memset they waited for the
+// whole fluid kernel beside them: memset nodes have no stream priority).
 __global__ void k_mesh_resolve(const GeomArgs a, int has_prev) {
     const bool inactive = slab_inactive(a);
     int lo[3], hi[3];
@@ -851,8 +854,15 @@ __global__ void k_mesh_resolve(const GeomArgs a, int has_prev) {
         if (a.b.live_list) {
             const int any = __syncthreads_or(live);
             const int lz = (int)blockIdx.z * kSlabZ + k;
-            if (any && linear_tid() == 0 && lz < a.bz)
-                a.b.live_list[atomicAdd(a.b.live_count, 1u)] = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * lz);
+            if (linear_tid() == 0 && lz < a.bz) {
+                const uint32_t block = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * lz);
+                if (any) {
+                    a.b.live_list[atomicAdd(a.b.live_count, 1u)] = block;
+                } else {
+                    a.b.block_counts[block] = 0;
+                    a.b.event_counts[block] = 0;
+                }
+            }
         }
     }
 }
@@ -1157,8 +1167,8 @@ __global__ void __launch_bounds__(256) k_link_count(const GeomArgs a) {
     count_block(a, blockIdx.x, blockIdx.y, blockIdx.z, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z),
                 wcount);
 }
-// The same over the live list of the mesh resolve (the other blocks' counts
-// are zeroed before): a fixed grid, list entry i to block i mod gridDim.x;
+// The same over the live list of the mesh resolve (which zeroed the other
+// blocks' counts): a fixed grid, list entry i to block i mod gridDim.x;
 // (gx, gy) are the box launch's grid extents.
 __global__ void __launch_bounds__(256) k_link_count_live(const GeomArgs a, int gx, int gy) {
     __shared__ uint32_t wcount[8];
@@ -1845,7 +1855,6 @@ void launch_classify(int geometry, int has_prev, const GridDesc& g, const FluidP
         const unsigned rblocks = (unsigned)(((int64_t)gb.ntris * 32 + 127) / 128);
         if (lean_raster) k_mesh_raster<1><<<rblocks, 128, 0, s>>>(a);
         else k_mesh_raster<0><<<rblocks, 128, 0, s>>>(a);
-        if (gb.live_list) cudaMemsetAsync(gb.live_count, 0, sizeof(uint32_t), s);
         k_mesh_resolve<<<sgrid, sblock, 0, s>>>(a, has_prev);
     }
 }
@@ -1866,8 +1875,6 @@ void launch_link_build(int geometry, int link_rule, const GridDesc& g, const Flu
     // with the mesh resolve's live list: count and emit over those blocks only
     const unsigned live_grid = (unsigned)std::min<int64_t>((int64_t)grid.x * grid.y * grid.z, 1024);
     if (gb.live_list) {
-        cudaMemsetAsync(gb.block_counts, 0, (size_t)gb.scan_blocks * sizeof(uint32_t), s);
-        cudaMemsetAsync(gb.event_counts, 0, (size_t)gb.scan_blocks * sizeof(uint32_t), s);
         k_link_count_live<<<live_grid, block, 0, s>>>(a, (int)grid.x, (int)grid.y);
     } else {
         k_link_count<<<grid, block, 0, s>>>(a);

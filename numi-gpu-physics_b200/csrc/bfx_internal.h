@@ -61,12 +61,11 @@ void launch_halo_values(int storage, const GridDesc& g, const FluidParams& fp, f
 // values from BulkArgs::face_dev).
 void launch_halo_yz(int storage, int rep_s, const GridDesc& g, const FluidParams& fp, const FluidBuffers& b,
                     cudaStream_t s);
-// The staged path's two launches (k_rare over the geometry box, then k_stream)
-// for callers that queue work between them; only for a simulation whose
-// population tensor map was encoded (16-bit storage, staged operator).
+// The two launches of a pipelined step (k_rare over the geometry box, then the
+// fluid cells) for callers that queue work between them.
 void launch_bulk_rare(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
                       const FluidBuffers& b, const int* box, cudaStream_t s);
-void launch_bulk_stream(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
+void launch_bulk_fluid(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
                         const FluidBuffers& b, const int* box, cudaStream_t s);
 // Block counts per segment of the two-level link-offset scan (bfx_geometry.cu).
 constexpr int kScanSegment = 8192;
