@@ -362,7 +362,7 @@ void encode_halo(bfx_sim* s, const FluidBuffers& fb, bool staged, cudaStream_t s
 void encode_link_build(bfx_sim* s, uint8_t* mprev, uint8_t* mnext, cudaStream_t st, cudaEvent_t lists_done = nullptr) {
     launch_link_build(s->cfg.geometry, s->cfg.link_rule, s->g, s->fp, s->box, geom_buffers(s, mprev, mnext), st,
                       lists_done);
-    s->launches += 5;
+    s->launches += link_build_launches(s->cfg.geometry, s->cfg.link_rule, s->fp, s->scan_blocks);
 }
 // The topology impulses of the step's events: they read the pre-step
 // populations, so they follow the previous step's fluid kernel and precede

@@ -914,46 +914,14 @@ __device__ float ellipsoid_link_fraction(const GeomArgs& a, int fx, int fy, int 
     return clampf(0.5f * (lo + hi), 1.0e-4f, 1.0f);
 }
 
-// min(d_A, d_B) - h, A and B the winning triangles of the two end cells.
-__device__ float mesh_ray_root(const GeomArgs& a, int fx, int fy, int fz, int sx, int sy, int sz) {
-    V3 fw = cell_world(a.fp, fx, fy, fz), sw = cell_world(a.fp, sx, sy, sz);
-    unsigned long long kf = box_key(a, fx, fy, fz), ks = box_key(a, sx, sy, sz);
-    uint32_t ta = (uint32_t)(ks & 0xFFFFFFFFull);
-    uint32_t tb = kf == 0xFFFFFFFFFFFFFFFFull ? ta : (uint32_t)(kf & 0xFFFFFFFFull);
-    if (ta >= a.b.ntris) return 0.5f;
-    if (tb >= a.b.ntris) tb = ta;
-    const float h = a.b.half_thickness;
-    float lo = 0.0f, hi = 1.0f;
-    bool found = false;
-    for (int i = 1; i <= 8; ++i) {
-        float t = (float)i * 0.125f;
-        V3 s = v3(mixf(fw.x, sw.x, t), mixf(fw.y, sw.y, t), mixf(fw.z, sw.z, t));
-        float gv = fminf(tri_distance(a, ta, s), tri_distance(a, tb, s)) - h;
-        if (gv <= 0.0f) {
-            hi = t;
-            found = true;
-            break;
-        }
-        lo = t;
-    }
-    if (!found) return 1.0f;
-    for (int it = 0; it < 24; ++it) {
-        float mid = 0.5f * (lo + hi);
-        V3 s = v3(mixf(fw.x, sw.x, mid), mixf(fw.y, sw.y, mid), mixf(fw.z, sw.z, mid));
-        float gv = fminf(tri_distance(a, ta, s), tri_distance(a, tb, s)) - h;
-        if (gv <= 0.0f) hi = mid;
-        else lo = mid;
-    }
-    return clampf(0.5f * (lo + hi), 1.0e-4f, 1.0f);
-}
-
-// mesh_ray_root on the 16 lanes of a group (gl: lane in the group, gmask: the
-// group's lanes in the warp).  The 8 march points, and in each of 8 rounds the
-// 7 midpoints of three bisection levels, are evaluated at once on separate
-// lanes -- two lanes per point, one per candidate triangle -- and the
-// decisions are then taken in the one-thread order.  Every evaluated point and
-// the returned fraction equal mesh_ray_root's; the search's dependent chain
-// shrinks from up to 32 distance evaluations to 9.
+// Root of min(d_A, d_B) - h on the link, A and B the winning triangles of the
+// two end cells: the first of 8 march points inside, then 24 bisections, on the
+// 16 lanes of a group (gl: lane in the group, gmask: the group's lanes in the
+// warp).  The 8 march points, and in each of 8 rounds the 7 midpoints of three
+// bisection levels, are evaluated at once on separate lanes -- two lanes per
+// point, one per candidate triangle -- and the decisions are then taken in the
+// order one thread would take them: the same points and the same fraction, with
+// a dependent chain of 9 distance evaluations instead of up to 32.
 __device__ float mesh_ray_root_group(const GeomArgs& a, int fx, int fy, int fz, int sx, int sy, int sz, int gl,
                                      unsigned gmask, int gshift) {
     V3 fw = cell_world(a.fp, fx, fy, fz), sw = cell_world(a.fp, sx, sy, sz);
@@ -1206,12 +1174,15 @@ __global__ void __launch_bounds__(128) k_topology(const GeomArgs a, int rep_s) {
 // counts (blockIdx.y 1) into block offsets, in two levels: k_scan_reduce sums
 // each segment of kScanSegment counts (a block per segment); k_scan_apply adds
 // the sums of the segments before its own and scans its segment (32
-// consecutive counts per thread).  Block 0 also sets the totals (and the link
-// list's overflow flag).  256-thread blocks: on the pipelined path they run
+// consecutive counts per thread).  With at most kScanDirect segments it adds the
+// counts before its segment itself, and k_scan_reduce (a launch of 2-4 us, more
+// than the extra reads) is left out.  The last block also sets the totals (and
+// the link list's overflow flag).  256-thread blocks: on the pipelined path they run
 // beside the persistent fluid kernel, in the registers it leaves free.
 // Integer sums: the offsets do not depend on the split.
 constexpr int kScanThreads = 256;
 constexpr int kScanPerThread = kScanSegment / kScanThreads;
+constexpr int kScanDirect = 2;
 __device__ __forceinline__ uint32_t block_sum_scan(uint32_t v, uint32_t* wtot) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -1237,27 +1208,19 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const GeomArgs a) 
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const GeomArgs a, int nseg) {
     __shared__ uint32_t wtot[kScanThreads / 32];
-    __shared__ uint32_t seg_base;
     const bool ev = blockIdx.y != 0;
     const uint32_t* counts = ev ? a.b.event_counts : a.b.block_counts;
     const uint32_t* sums = ev ? a.b.event_sums : a.b.scan_sums;
     uint32_t* offsets = ev ? a.b.event_offsets : a.b.block_offsets;
     const int nb = a.b.scan_blocks;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) {
-        uint32_t b = 0;
-        for (int k = 0; k < (int)blockIdx.x; ++k) b += sums[k];
-        seg_base = b;
-        if (blockIdx.x == 0) {
-            uint64_t total = 0;
-            for (int k = 0; k < nseg; ++k) total += sums[k];
-            if (ev) {
-                *a.b.event_total = (uint32_t)total;  // at most one event a box cell
-            } else {
-                a.b.state->link_count = (int64_t)total;
-                a.b.state->link_overflow = total > a.b.link_capacity ? 1u : 0u;
-            }
-        }
+    uint32_t before = 0;  // the counts before this segment
+    if (nseg <= kScanDirect) {
+        for (int i = threadIdx.x; i < (int)blockIdx.x * kScanSegment; i += kScanThreads) before += counts[i];
+        before = block_sum_scan(before, wtot);
+        __syncthreads();
+    } else {
+        for (int k = 0; k < (int)blockIdx.x; ++k) before += sums[k];
     }
     // kScanPerThread consecutive counts per thread
     const int first = blockIdx.x * kScanSegment + kScanPerThread * threadIdx.x;
@@ -1276,9 +1239,18 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const GeomArgs a, i
     }
     if (lane == 31) wtot[warp] = incl;
     __syncthreads();
-    uint32_t base = seg_base;
+    uint32_t base = before;
     for (int w = 0; w < warp; ++w) base += wtot[w];
     base += incl - mine;
+    if ((int)blockIdx.x == nseg - 1 && threadIdx.x == kScanThreads - 1) {
+        const uint32_t total = base + mine;
+        if (ev) {
+            *a.b.event_total = total;  // at most one event a box cell
+        } else {
+            a.b.state->link_count = (int64_t)total;
+            a.b.state->link_overflow = total > a.b.link_capacity ? 1u : 0u;
+        }
+    }
 #pragma unroll
     for (int k = 0; k < kScanPerThread; ++k) {
         if (first + k < nb) offsets[first + k] = base;
@@ -1286,11 +1258,19 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const GeomArgs a, i
     }
 }
 
+// Linear link rule (BF.metal:2044-2076): fluid distance fd >= 0, solid distance sd <= 0.
+__device__ __forceinline__ float linear_fraction(float fd, float sd) {
+    return clampf(fd / fmaxf(fd - sd, 1.0e-6f), 1.0e-4f, 1.0f);
+}
+
 // Cut-link and event compaction: every persistent fluid cell appends its
 // links (in direction order) at the block offset plus the shuffle prefix of
 // the preceding threads, so the list is ordered by box cell then direction;
 // every event cell appends itself to the event list in box-cell order.
-__device__ __forceinline__ void emit_block(const GeomArgs& a, int bxi, int byi, int bzi, int block, uint32_t* wsum) {
+// fraction: 0 none (a search kernel follows), 1 halfway links (1/2), 2 the
+// mesh's linear rule; writing those here saves the launch over the link list.
+__device__ __forceinline__ void emit_block(const GeomArgs& a, int bxi, int byi, int bzi, int block, uint32_t* wsum,
+                                           int fraction) {
     // blocks without links or events (most of the box) emit nothing; the
     // others were counted, so their active cells' bits are this step's
     if (a.b.block_counts[block] == 0 && a.b.event_counts[block] == 0) return;
@@ -1323,38 +1303,41 @@ __device__ __forceinline__ void emit_block(const GeomArgs& a, int bxi, int byi, 
     if (event) a.b.event_cell[a.b.event_offsets[block] + (excl >> 16)] = (uint32_t)gid;
     if (mine == 0) return;
     uint32_t pos = a.b.block_offsets[block] + (excl & 0xFFFFu);
+    const float fd = fraction == 2 ? fmaxf(a.b.wall[gid].w, 0.0f) : 0.0f;
 #pragma unroll
     for (int q = 1; q < 19; ++q) {
         if (!(bits & (1u << q))) continue;
         if (pos < a.b.link_capacity) {
             int sx = x - cx(q), sy = y - cy(q), sz = z - cz(q);
             wrap(g, sx, sy, sz);  // inside: the source is solid
+            const int64_t src = flat(g, sx, sy, sz);
             a.b.link_cell[pos] = (uint32_t)gid;
-            a.b.link_meta[pos] = (uint32_t)q | ((uint32_t)(a.b.mask_next[flat(g, sx, sy, sz)] & kPartMask) << 8);
+            a.b.link_meta[pos] = (uint32_t)q | ((uint32_t)(a.b.mask_next[src] & kPartMask) << 8);
+            if (fraction == 1) a.b.link_q[pos] = 0.5f;
+            if (fraction == 2) a.b.link_q[pos] = linear_fraction(fd, fminf(a.b.wall[src].w, 0.0f));
         }
         ++pos;
     }
 }
-__global__ void __launch_bounds__(256) k_links_emit(const GeomArgs a) {
+__global__ void __launch_bounds__(256) k_links_emit(const GeomArgs a, int fraction) {
     __shared__ uint32_t wsum[8];
     emit_block(a, blockIdx.x, blockIdx.y, blockIdx.z, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z),
-               wsum);
+               wsum, fraction);
 }
 // The same over the live list (k_link_count_live).
-__global__ void __launch_bounds__(256) k_links_emit_live(const GeomArgs a, int gx, int gy) {
+__global__ void __launch_bounds__(256) k_links_emit_live(const GeomArgs a, int gx, int gy, int fraction) {
     __shared__ uint32_t wsum[8];
     const uint32_t n = *a.b.live_count;
     for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
         const int b = (int)a.b.live_list[i];
-        emit_block(a, b % gx, (b / gx) % gy, b / (gx * gy), b, wsum);
+        emit_block(a, b % gx, (b / gx) % gy, b / (gx * gy), b, wsum, fraction);
         __syncthreads();
     }
 }
 
-// Link fractions, one thread per emitted link (the bisections and ray roots
-// are long and occur only at the surface: a thread per box cell would leave
-// most lanes idle while a few run them).
-__global__ void __launch_bounds__(128) k_links_fraction(const GeomArgs a, int geometry, int link_rule, int interpolated) {
+// Bisected link fractions of the analytic shapes, one thread per emitted link
+// (a thread per box cell would leave most lanes idle while a few run them).
+__global__ void __launch_bounds__(128) k_links_fraction(const GeomArgs a, int geometry) {
     const Grid& g = a.g;
     int64_t count = a.b.state->link_count;
     if (count > (int64_t)a.b.link_capacity) count = a.b.link_capacity;
@@ -1365,22 +1348,9 @@ __global__ void __launch_bounds__(128) k_links_fraction(const GeomArgs a, int ge
         unflat(g, gid, x, y, z);
         int sx = x - cx(q), sy = y - cy(q), sz = z - cz(q);
         float qf = 0.5f;
-        if (interpolated && wrap(g, sx, sy, sz)) {
-            const int64_t s = flat(g, sx, sy, sz);
-            if (geometry == BFX_GEOMETRY_ELLIPSOID) {
-                qf = ellipsoid_link_fraction(a, x, y, z, sx, sy, sz);
-            } else if (geometry == BFX_GEOMETRY_FLAPPING_WING) {
-                qf = wing_link_fraction(a, q, sx, sy, sz);
-            } else if (geometry == BFX_GEOMETRY_MESH) {
-                if (link_rule == BFX_LINK_RAY_ROOT) {
-                    qf = mesh_ray_root(a, x, y, z, sx, sy, sz);
-                } else {
-                    float sd = fminf(a.b.wall[s].w, 0.0f);
-                    float fd = fmaxf(a.b.wall[gid].w, 0.0f);
-                    qf = clampf(fd / fmaxf(fd - sd, 1.0e-6f), 1.0e-4f, 1.0f);
-                }
-            }
-        }
+        if (wrap(g, sx, sy, sz))
+            qf = geometry == BFX_GEOMETRY_ELLIPSOID ? ellipsoid_link_fraction(a, x, y, z, sx, sy, sz)
+                                                    : wing_link_fraction(a, q, sx, sy, sz);
         a.b.link_q[i] = qf;
     }
 }
@@ -1867,6 +1837,18 @@ void launch_classify(int geometry, int has_prev, const GridDesc& g, const FluidP
     default: FN<StoreF32>(__VA_ARGS__); break;                             \
     }
 
+// The link fractions a search kernel finds: a ray root, or a bisection.
+static bool ray_links(int geometry, int link_rule, const FluidParams& fp) {
+    return geometry == BFX_GEOMETRY_MESH && link_rule == BFX_LINK_RAY_ROOT && fp.interpolated;
+}
+static bool bisected_links(int geometry, const FluidParams& fp) {
+    return fp.interpolated && (geometry == BFX_GEOMETRY_ELLIPSOID || geometry == BFX_GEOMETRY_FLAPPING_WING);
+}
+int link_build_launches(int geometry, int link_rule, const FluidParams& fp, int scan_blocks) {
+    const int nseg = (scan_blocks + kScanSegment - 1) / kScanSegment;
+    return 3 + (nseg > kScanDirect) + (ray_links(geometry, link_rule, fp) || bisected_links(geometry, fp));
+}
+
 void launch_link_build(int geometry, int link_rule, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,
                        const GeomBuffers& gb, cudaStream_t s, cudaEvent_t lists_done) {
     GeomArgs a = make_geom(g, fp, box, gb, nullptr);
@@ -1880,19 +1862,22 @@ void launch_link_build(int geometry, int link_rule, const GridDesc& g, const Flu
         k_link_count<<<grid, block, 0, s>>>(a);
     }
     const int nseg = (a.b.scan_blocks + kScanSegment - 1) / kScanSegment;
-    k_scan_reduce<<<dim3(nseg, 2), kScanThreads, 0, s>>>(a);
+    if (nseg > kScanDirect) k_scan_reduce<<<dim3(nseg, 2), kScanThreads, 0, s>>>(a);
     k_scan_apply<<<dim3(nseg, 2), kScanThreads, 0, s>>>(a, nseg);
-    if (gb.live_list) k_links_emit_live<<<live_grid, block, 0, s>>>(a, (int)grid.x, (int)grid.y);
-    else k_links_emit<<<grid, block, 0, s>>>(a);
+    const bool ray = ray_links(geometry, link_rule, fp), bisect = bisected_links(geometry, fp);
+    const int fraction = ray || bisect ? 0 : (fp.interpolated && geometry == BFX_GEOMETRY_MESH ? 2 : 1);
+    if (gb.live_list) k_links_emit_live<<<live_grid, block, 0, s>>>(a, (int)grid.x, (int)grid.y, fraction);
+    else k_links_emit<<<grid, block, 0, s>>>(a, fraction);
     if (lists_done) cudaEventRecord(lists_done, s);
-    if (geometry == BFX_GEOMETRY_MESH && link_rule == BFX_LINK_RAY_ROOT && fp.interpolated) {
+    if (ray) {
         const unsigned rblocks =
             (unsigned)std::max<int64_t>(1, std::min<int64_t>(4096, ((int64_t)gb.link_capacity * 16 + 127) / 128));
         k_links_fraction_ray<<<rblocks, 128, 0, s>>>(a);
-        return;
+    } else if (bisect) {
+        const unsigned fblocks =
+            (unsigned)std::max<int64_t>(1, std::min<int64_t>(4096, ((int64_t)gb.link_capacity + 127) / 128));
+        k_links_fraction<<<fblocks, 128, 0, s>>>(a, geometry);
     }
-    const unsigned fblocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(4096, ((int64_t)gb.link_capacity + 127) / 128));
-    k_links_fraction<<<fblocks, 128, 0, s>>>(a, geometry, link_rule, fp.interpolated);
 }
 
 template <class S>

@@ -169,6 +169,8 @@ void launch_classify(int geometry, int has_prev, const GridDesc& g, const FluidP
 // link fractions.
 void launch_link_build(int geometry, int link_rule, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,
                        const GeomBuffers& gb, cudaStream_t s, cudaEvent_t lists_done = nullptr);
+// Kernel launches of one launch_link_build call.
+int link_build_launches(int geometry, int link_rule, const FluidParams& fp, int scan_blocks);
 // Topology impulses of the event list into topo_partials; reads the pre-step
 // populations, so it runs before the link kernel writes any.
 void launch_topology(int storage, int rep_s, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,
