@@ -270,6 +270,7 @@ GeomBuffers geom_buffers(bfx_sim* s, uint8_t* mprev, uint8_t* mnext) {
     b.event_total = s->event_total;
     // the occupancy test hook's replayed masks are not what the resolve saw
     b.live_list = s->topo_mode ? nullptr : s->live_list;
+    b.open_bounds = s->topo_mode != 0;
     b.live_count = s->live_count;
     b.cell_bits = s->cell_bits;
     b.box_blocks = s->box_blocks;
@@ -865,9 +866,11 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
     // A mesh touches cells within the raster guard (half thickness + 2 cells)
     // of its vertices' bounding box; three more cells cover the cells solid or
     // flagged in the two previous steps (bounded motion, Mach <= 0.25).
+    // The prescribed wing's bounds hold its solid cells of both steps: one cell
+    // more for the cut links' fluid ends, two for rounding.
     fp.act_margin = c.geometry == BFX_GEOMETRY_MESH
                         ? (int)std::ceil(c.mesh_half_thickness / c.cell_size) + 2 + 3
-                        : 0;
+                        : (c.geometry == BFX_GEOMETRY_FLAPPING_WING ? 3 : 0);
 
     s->inline_faces = bulk_inline_faces(c.storage, g, fp, c.geometry != BFX_GEOMETRY_NONE);
     if (s->inline_faces) s->faces = make_face_equilibria(fp);

@@ -142,6 +142,7 @@ struct GeomBuffers {
     const float* kf_times;          // keyframe replay: times, frames x vertices x 3 offsets (kf_count >= 2)
     const float* kf_points;
     int kf_count;
+    int open_bounds;                // the whole geometry box is active (occupancy test hook)
     uint32_t* live_list;            // box blocks with a key or an occupancy change (mesh resolve), or null
     uint32_t* live_count;           // [1] entries in live_list
     uint32_t* cell_bits;            // per box cell of a counted block: link sources (bits 1-18), event (bit 0)
