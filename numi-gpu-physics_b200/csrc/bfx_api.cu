@@ -93,6 +93,7 @@ struct bfx_sim {
     int kf_count = 0;
     uint32_t* mesh_tris = nullptr;
     uint8_t* mesh_tri_part = nullptr;
+    uint4* mesh_order = nullptr;
     float4* mesh_pos = nullptr;
     float4* mesh_vel = nullptr;
     unsigned long long* keys = nullptr;
@@ -250,6 +251,7 @@ GeomBuffers geom_buffers(bfx_sim* s, uint8_t* mprev, uint8_t* mnext) {
     b.kf_count = s->kf_count;
     b.mesh_tris = s->mesh_tris;
     b.mesh_tri_part = s->mesh_tri_part;
+    b.mesh_order = s->mesh_order;
     b.mesh_pos = s->mesh_pos;
     b.mesh_vel = s->mesh_vel;
     b.keys = s->keys;
@@ -299,16 +301,25 @@ struct TapeSlot {
     float* link_tangent;    // per-link tangent scratch shared by all slots
 };
 
-// Classification for the geometry at the current state (pose and frames,
-// occupancy, wall field, mesh keys), on the simulation's stream or another.
-void encode_geometry_build(bfx_sim* s, int init, uint8_t* mprev, uint8_t* mnext, cudaStream_t st = nullptr) {
+// Classification for the geometry at the current state, in two parts: the pose
+// and a mesh's raster keys, then occupancy and wall field; on the simulation's
+// stream or another.
+void encode_pose(bfx_sim* s, int init, uint8_t* mprev, uint8_t* mnext, cudaStream_t st) {
     GeomBuffers gb = geom_buffers(s, mprev, mnext);
-    if (!st) st = s->stream;
     launch_prepare(s->cfg.geometry, s->cfg.time_step, s->g, s->fp, s->box, gb, init, st);
-    // beside the TRT staged kernel (pipelined build): the register-lean raster
-    const bool lean = st == s->side && s->tma_ok && s->cfg.collision == BFX_COLLISION_TRT;
-    launch_classify(s->cfg.geometry, init ? 0 : 1, s->g, s->fp, s->box, gb, st, lean);
-    s->launches += 1 + (s->cfg.geometry == BFX_GEOMETRY_MESH ? 4 : 1);
+    s->launches += 1;
+    if (s->cfg.geometry == BFX_GEOMETRY_MESH) {
+        launch_mesh_keys(s->g, s->fp, s->box, gb, st);
+        s->launches += 3;
+    }
+}
+void encode_classify(bfx_sim* s, int init, uint8_t* mprev, uint8_t* mnext, cudaStream_t st) {
+    launch_classify(s->cfg.geometry, init ? 0 : 1, s->g, s->fp, s->box, geom_buffers(s, mprev, mnext), st);
+    s->launches += 1;
+}
+void encode_geometry_build(bfx_sim* s, int init, uint8_t* mprev, uint8_t* mnext) {
+    encode_pose(s, init, mprev, mnext, s->stream);
+    encode_classify(s, init, mprev, mnext, s->stream);
 }
 
 // The next step's geometry build can overlap this step's fluid kernel: the
@@ -503,9 +514,17 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     if (pipelined) {
         // Beside the fluid kernel, on the side stream: the next step's
         // geometry (masks swap roles) and its cut-link and event lists.
+        // Beside the staged kernel, which saturates the memory, the issue slots
+        // and the instruction fetch, the chain's first kernels take 6-8 times as
+        // long as alone (pose 57 against 7 us, vertices 8 against 3, keys 22
+        // against 3, raster 400 against 50), longer than the fluid kernel lasts:
+        // they go before the fork there, and the rest fits beside it.
+        const bool early = s->tma_ok;
+        if (early) encode_pose(s, 0, mnext, mprev, s->stream);
         cudaEventRecord(s->fork_ev, s->stream);
         cudaStreamWaitEvent(s->side, s->fork_ev, 0);
-        encode_geometry_build(s, 0, mnext, mprev, s->side);
+        if (!early) encode_pose(s, 0, mnext, mprev, s->side);
+        encode_classify(s, 0, mnext, mprev, s->side);
         if (s->geometry()) encode_link_build(s, mnext, mprev, s->side, s->lists_ev);
         else cudaEventRecord(s->lists_ev, s->side);
         cudaEventRecord(s->join_ev, s->side);
@@ -720,6 +739,53 @@ float geometry_radius(const bfx_config* c, const bfx_bird* b, const bfx_mesh* m)
         r = std::max(r, d);
     }
     return r + c->mesh_half_thickness + 2.0f * c->cell_size;
+}
+
+// The triangles (vertices, id) in the order the raster takes them: along a Morton curve of the
+// centroid within each segment (10 bits an axis of the segment-frame
+// coordinates, the first keyframe's for a replay), every eighth triangle of the
+// curve first.  Those leave a key near the final one in almost every voxel,
+// which lets the others drop most of theirs; the order changes no result.
+std::vector<uint4> raster_order(const bfx_mesh* m) {
+    const float* pts = m->keyframe_count >= 2 ? m->keyframe_points : m->local_vertices;
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (uint32_t i = 0; i < m->vertex_count; ++i)
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = std::min(lo[k], pts[3 * i + k]);
+            hi[k] = std::max(hi[k], pts[3 * i + k]);
+        }
+    // one scale for the three axes, so that the curve's cells are cubes
+    const float extent = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
+    const float scale = extent > 0.0f ? 1023.0f / (3.0f * extent) : 0.0f;
+    auto spread = [](uint32_t v) {
+        uint64_t r = 0;
+        for (int b = 0; b < 10; ++b) r |= (uint64_t)((v >> b) & 1u) << (3 * b);
+        return r;
+    };
+    std::vector<std::pair<uint64_t, uint32_t>> keyed(m->triangle_count);
+    for (uint32_t t = 0; t < m->triangle_count; ++t) {
+        const uint32_t* v = m->triangles + 3 * t;
+        uint64_t code = (uint64_t)m->vertex_segment[v[0]] << 32;
+        for (int k = 0; k < 3; ++k) {
+            const float c = (pts[3 * v[0] + k] - lo[k]) + (pts[3 * v[1] + k] - lo[k]) + (pts[3 * v[2] + k] - lo[k]);
+            const float f = c * scale;
+            const uint32_t i = f >= 0.0f ? (uint32_t)std::min(f, 1023.0f) : 0u;  // a NaN counts as 0
+            code |= spread(i) << k;
+        }
+        keyed[t] = {code, t};
+    }
+    std::sort(keyed.begin(), keyed.end());
+    std::vector<uint4> order;
+    order.reserve(m->triangle_count);
+    auto append = [&](uint32_t i) {
+        const uint32_t t = keyed[i].second;
+        const uint32_t* v = m->triangles + 3 * (size_t)t;
+        order.push_back(make_uint4(v[0], v[1], v[2], t));
+    };
+    for (uint32_t i = 0; i < m->triangle_count; i += 8) append(i);
+    for (uint32_t i = 0; i < m->triangle_count; ++i)
+        if (i % 8 != 0) append(i);
+    return order;
 }
 
 }  // namespace
@@ -996,6 +1062,10 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
             cudaMemcpyAsync(s->mesh_tris, mesh->triangles, (size_t)s->ntris * 3 * sizeof(uint32_t),
                             cudaMemcpyHostToDevice, s->stream);
             cudaMemcpyAsync(s->mesh_tri_part, mesh->triangle_part, s->ntris, cudaMemcpyHostToDevice, s->stream);
+            const std::vector<uint4> order = raster_order(mesh);
+            BFX_ALLOC(s->mesh_order, (size_t)s->ntris * sizeof(uint4));
+            cudaMemcpyAsync(s->mesh_order, order.data(), (size_t)s->ntris * sizeof(uint4), cudaMemcpyHostToDevice,
+                            s->stream);
             if (mesh->keyframe_count >= 2) {
                 s->kf_count = (int)mesh->keyframe_count;
                 const size_t np = (size_t)s->kf_count * s->nverts * 3;

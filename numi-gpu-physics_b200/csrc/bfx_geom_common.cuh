@@ -226,6 +226,38 @@ __device__ __forceinline__ V3 closest_point(V3 p, V3 a, V3 b, V3 c, V3& bary) {
     return v3(a.x + ab.x * v + ac.x * w, a.y + ab.y * v + ac.y * w, a.z + ab.z * v + ac.z * w);
 }
 
+// |p - closest_point(p)| without branches: the region is decided by the same
+// comparisons in the same order, and its one division, edge and base point are
+// selected, so the value equals closest_point's bit for bit (an unused term
+// adds a zero).  A warp whose lanes fall in different regions runs one path
+// instead of up to seven, each with its own division.
+__device__ __forceinline__ float closest_distance(V3 p, V3 a, V3 b, V3 c) {
+    const V3 ab = b - a, ac = c - a, ap = p - a, bp = p - b, cp = p - c;
+    const float d1 = dot(ab, ap), d2 = dot(ac, ap), d3 = dot(ab, bp), d4 = dot(ac, bp), d5 = dot(ab, cp),
+                d6 = dot(ac, cp);
+    const float vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
+    const bool in_a = d1 <= 0.0f && d2 <= 0.0f;
+    const bool in_b = d3 >= 0.0f && d4 <= d3;
+    const bool on_ab = vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f;
+    const bool in_c = d6 >= 0.0f && d5 <= d6;
+    const bool on_ac = vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f;
+    const bool on_bc = va <= 0.0f && (d4 - d3) >= 0.0f && (d5 - d6) >= 0.0f;
+    // 0 a, 1 b, 2 ab, 3 c, 4 ac, 5 bc, 6 face
+    const int r = in_a ? 0 : (in_b ? 1 : (on_ab ? 2 : (in_c ? 3 : (on_ac ? 4 : (on_bc ? 5 : 6)))));
+    const float num = r == 2 ? d1 : (r == 4 ? d2 : (r == 5 ? d4 - d3 : 1.0f));
+    const float den = r == 2 ? d1 - d3
+                             : (r == 4 ? d2 - d6
+                                       : (r == 5 ? (d4 - d3) + (d5 - d6) : (r == 6 ? fmaxf(va + vb + vc, 1.0e-20f) : 1.0f)));
+    const float quot = num / den;
+    const float s = r == 6 ? vb * quot : (r == 2 || r == 4 || r == 5 ? quot : 0.0f);
+    const float t = r == 6 ? vc * quot : 0.0f;
+    const V3 base = r == 1 || r == 5 ? b : (r == 3 ? c : a);
+    const V3 e = r == 4 ? ac : (r == 5 ? c - b : ab);
+    const V3 d = v3(p.x - (base.x + e.x * s + ac.x * t), p.y - (base.y + e.y * s + ac.y * t),
+                    p.z - (base.z + e.z * s + ac.z * t));
+    return length(d);
+}
+
 // Articulated vertex placement: segment 0 rides the body frame, 1 / 2 the left
 // / right wing frames (the indexed surface preparation of BF.metal:1589-1622,
 
@@ -277,10 +309,9 @@ __device__ __forceinline__ uint32_t link_sources(const Grid& g, const uint8_t* m
 // Ten-iteration bisection from the fluid node toward the solid node on the
 
 __device__ __forceinline__ float tri_distance(const GeomArgs& a, uint32_t t, V3 w) {
-    V3 A, B, C, bary;
+    V3 A, B, C;
     tri_vertices(a, t, A, B, C);
-    V3 cp = closest_point(w, A, B, C, bary);
-    return length(w - cp);
+    return closest_distance(w, A, B, C);
 }
 
 __device__ __forceinline__ unsigned long long box_key(const GeomArgs& a, int x, int y, int z) {

@@ -760,102 +760,247 @@ __global__ void k_mesh_clear(const GeomArgs a) {
     }
 }
 
-// One warp per triangle: the lanes share the triangle's voxel box (its AABB
-// grown by the half thickness plus two cells, clamped to the lattice and the
-// geometry box) and each keeps the atomic minimum of (quantised distance,
-// triangle id) per voxel.  LEAN caps a thread at 40 registers (a few bytes
-// spill): the pipelined build runs the raster beside the persistent TRT fluid
-// kernel, whose CTA leaves about 22 K registers of an SM free, room for four
-// lean blocks against two of the unconstrained (64-register) kernel.
-template <int LEAN>
-__global__ void __launch_bounds__(128, LEAN ? 12 : 1) k_mesh_raster(const GeomArgs a) {
-    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// Triangle raster: the atomic minimum of (quantised distance, triangle id) per
+// voxel over each triangle's voxel box (its AABB grown by the half thickness
+// plus two cells, clamped to the lattice and the geometry box).  Voxels farther
+// than that guard from the triangle decide nothing (a cell next to a solid one
+// lies within h + sqrt(3) dx of its triangle, inside the guard), so only voxels
+// within the guard of the triangle's bounding sphere are candidates.
+//
+// Bound by instruction issue: a fine mesh has some 160 candidates per triangle
+// and its exact distance costs about 200 instructions.  So a candidate is
+// dropped when the triangle cannot lower the key found there:
+//   - the triangle lies in a disc of radius r and half thickness `thick` about
+//     its centroid, normal to its own normal; at height |h| and lateral distance
+//     `lat` from the centroid its distance is at least
+//     sqrt((|h| - thick)^2 + (lat - r)^2).  With final keys that leaves 5 of the
+//     158 candidates of a 0.4 x 0.5 cell triangle on a flat plate (centroid
+//     distance minus r would leave 27);
+//   - every eighth triangle along a Morton curve comes first (mesh_order), so
+//     most triangles find keys near their final values;
+//   - the bound carries a slack that covers rounding and the key's quantum, so
+//     ties still go to the smallest id.
+// And the lanes are kept busy: a warp takes up to kRasterTris triangles (a lane
+// prepares each), lists the (x, y) columns of their spheres together, and hands
+// every column to two lanes that walk its z range, four keys in flight each;
+// what is left is queued, so that the distance search runs on full warps,
+// without branches (closest_distance).  Keys are minima, so the order of the
+// atomics changes no result.
+// 145 k triangles (768 x 384 x 384 bird) 407 -> 278 us against one warp per
+// triangle over every voxel of its box; 16 k triangles 50 -> 52 us: there the
+// whole mesh is in flight at once and finds no keys to drop by.
+constexpr int kRasterTris = 4;
+struct RasterTri {
+    float cen[3], reach2;
+    float nrm[3], thick;
+    float disc, slack;
+    int lo[3], ext[3];
+    uint32_t id;
+    float vert[9];
+    int _pad;               // 27 words: the four records start on different banks
+};
+struct RasterWarp {
+    RasterTri tri[kRasterTris];
+    int4 column[48];        // x, y, first z, z count | triangle << 28
+    float2 offset[48];      // x, y distance from the centroid
+    int4 queue[64];         // x, y, z, triangle
+};
+// square root to about 1e-6 (the bound's slack covers it)
+__device__ __forceinline__ float approx_sqrt(float v) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+__global__ void __launch_bounds__(128, 8) k_mesh_raster(const GeomArgs a, int per_warp) {
+    __shared__ RasterWarp warps[4];
     const int lane = threadIdx.x & 31;
-    if (t >= a.b.ntris) return;
-    V3 A, B, C;
-    tri_vertices(a, t, A, B, C);
+    RasterWarp& w = warps[threadIdx.x >> 5];
+    const uint32_t first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (uint32_t)per_warp;
+    if (first >= a.b.ntris) return;
+    const int count = a.b.ntris - first < (uint32_t)per_warp ? (int)(a.b.ntris - first) : per_warp;
     const float cs = a.fp.dx;
     const float guard = a.b.half_thickness + 2.0f * cs;
-    int lo[3], hi[3];
-    const int dims[3] = {a.g.nx, a.g.ny, a.g.nz};
-    const int ext[3] = {a.bx, a.by, a.bz};
-    const int32_t* o = a.b.state->box_origin;
-    float mn[3] = {fminf(A.x, fminf(B.x, C.x)), fminf(A.y, fminf(B.y, C.y)), fminf(A.z, fminf(B.z, C.z))};
-    float mx[3] = {fmaxf(A.x, fmaxf(B.x, C.x)), fmaxf(A.y, fmaxf(B.y, C.y)), fmaxf(A.z, fmaxf(B.z, C.z))};
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = (int)floorf(((mn[k] - guard) - a.fp.origin[k]) / cs - 0.5f);
-        hi[k] = (int)ceilf(((mx[k] + guard) - a.fp.origin[k]) / cs - 0.5f);
-        lo[k] = lo[k] < 0 ? 0 : (lo[k] > dims[k] - 1 ? dims[k] - 1 : lo[k]);
-        hi[k] = hi[k] < 0 ? 0 : (hi[k] > dims[k] - 1 ? dims[k] - 1 : hi[k]);
-        // confine to the geometry box (the key array is box-local)
-        lo[k] = lo[k] < o[k] ? o[k] : lo[k];
-        hi[k] = hi[k] > o[k] + ext[k] - 1 ? o[k] + ext[k] - 1 : hi[k];
+    const int ox = a.b.state->box_origin[0], oy = a.b.state->box_origin[1], oz = a.b.state->box_origin[2];
+    if (lane < count) {
+        RasterTri& r = w.tri[lane];
+        const uint4 tri = a.b.mesh_order[first + lane];
+        const V3 A = v3(a.b.mesh_pos[tri.x]), B = v3(a.b.mesh_pos[tri.y]), C = v3(a.b.mesh_pos[tri.z]);
+        const int dims[3] = {a.g.nx, a.g.ny, a.g.nz};
+        const int box[3] = {a.bx, a.by, a.bz};
+        const int o[3] = {ox, oy, oz};
+        const float mn[3] = {fminf(A.x, fminf(B.x, C.x)), fminf(A.y, fminf(B.y, C.y)), fminf(A.z, fminf(B.z, C.z))};
+        const float mx[3] = {fmaxf(A.x, fmaxf(B.x, C.x)), fmaxf(A.y, fmaxf(B.y, C.y)), fmaxf(A.z, fmaxf(B.z, C.z))};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            int lo = (int)floorf(((mn[k] - guard) - a.fp.origin[k]) / cs - 0.5f);
+            int hi = (int)ceilf(((mx[k] + guard) - a.fp.origin[k]) / cs - 0.5f);
+            lo = lo < 0 ? 0 : (lo > dims[k] - 1 ? dims[k] - 1 : lo);
+            hi = hi < 0 ? 0 : (hi > dims[k] - 1 ? dims[k] - 1 : hi);
+            // confine to the geometry box (the key array is box-local)
+            lo = lo < o[k] ? o[k] : lo;
+            hi = hi > o[k] + box[k] - 1 ? o[k] + box[k] - 1 : hi;
+            r.lo[k] = lo;
+            r.ext[k] = hi - lo + 1;
+        }
+        // the bounding sphere about the centroid, with a relative slack that
+        // covers the rounding of the squared distances
+        const V3 cen = v3((A.x + B.x + C.x) * (1.0f / 3.0f), (A.y + B.y + C.y) * (1.0f / 3.0f),
+                          (A.z + B.z + C.z) * (1.0f / 3.0f));
+        const float r2 = fmaxf(dot(A - cen, A - cen), fmaxf(dot(B - cen, B - cen), dot(C - cen, C - cen)));
+        const float radius = sqrtf(r2);
+        const float reach = radius + guard;
+        r.reach2 = reach * reach * 1.0001f;
+        // coordinate rounding of this size, and the key's quantum
+        const float slack = 1.0e-3f * cs + 4.0e-6f * (fabsf(cen.x) + fabsf(cen.y) + fabsf(cen.z));
+        // unit normal; zero for a degenerate triangle, whose bound is then the sphere's
+        V3 nrm = cross(B - A, C - A);
+        const float n2 = dot(nrm, nrm);
+        nrm = nrm * (n2 > 1.0e-30f ? rsqrtf(n2) : 0.0f);
+        r.thick = fmaxf(fabsf(dot(nrm, A - cen)), fmaxf(fabsf(dot(nrm, B - cen)), fabsf(dot(nrm, C - cen)))) + 0.1f * slack;
+        r.disc = radius * 1.0001f + slack;
+        r.slack = slack;
+        r.cen[0] = cen.x;
+        r.cen[1] = cen.y;
+        r.cen[2] = cen.z;
+        r.nrm[0] = nrm.x;
+        r.nrm[1] = nrm.y;
+        r.nrm[2] = nrm.z;
+        r.id = tri.w;
+        r.vert[0] = A.x;
+        r.vert[1] = A.y;
+        r.vert[2] = A.z;
+        r.vert[3] = B.x;
+        r.vert[4] = B.y;
+        r.vert[5] = B.z;
+        r.vert[6] = C.x;
+        r.vert[7] = C.y;
+        r.vert[8] = C.z;
     }
-    const int ex = hi[0] - lo[0] + 1, ey = hi[1] - lo[1] + 1, ez = hi[2] - lo[2] + 1;
-    if (ex <= 0 || ey <= 0 || ez <= 0) return;
-    const int total = ex * ey * ez;
-    // Voxels farther than the guard from the triangle decide nothing (a cell
-    // next to a solid one lies within h + sqrt(3) dx of its triangle, inside
-    // the guard), so only voxels within the guard of the triangle's bounding
-    // sphere compute their distance: a superset, with a relative slack that
-    // covers the rounding of the squared distances.
-    const V3 cen = v3((A.x + B.x + C.x) * (1.0f / 3.0f), (A.y + B.y + C.y) * (1.0f / 3.0f),
-                      (A.z + B.z + C.z) * (1.0f / 3.0f));
-    const float r2 = fmaxf(dot(A - cen, A - cen), fmaxf(dot(B - cen, B - cen), dot(C - cen, C - cen)));
-    const float reach = sqrtf(r2) + guard;
-    const float reach2 = reach * reach * 1.0001f;
-    // voxel index -> (x, y, z) by reciprocal multiplication (exact for these small extents)
-    const float inv_ex = 1.0f / (float)ex, inv_ey = 1.0f / (float)ey;
-    auto voxel = [&](int i, int& x, int& y, int& z) {
-        const int r = (int)(((float)i + 0.5f) * inv_ex);
-        const int zi = (int)(((float)r + 0.5f) * inv_ey);
-        x = lo[0] + (i - r * ex);
-        y = lo[1] + (r - zi * ey);
-        z = lo[2] + zi;
-    };
-    auto key_voxel = [&](int i) {
-        int x, y, z;
-        voxel(i, x, y, z);
-        V3 w = cell_world(a.fp, x, y, z), bary;
-        V3 cp = closest_point(w, A, B, C, bary);
-        float dc = length(w - cp) / cs;
-        float bin = roundf(dc * 65536.0f);
-        unsigned long long ub = bin >= 4294967295.0f ? 0xFFFFFFFFull : (unsigned long long)bin;
-        unsigned long long key = (ub << 32) | (unsigned long long)t;
-        int64_t bi = (int64_t)(x - o[0]) + (int64_t)a.bx * ((int64_t)(y - o[1]) + (int64_t)a.by * (z - o[2]));
-        atomicMin(&a.b.keys[bi], key);
-    };
-    // The sphere test rejects a good share of the box: queue the voxels that
-    // pass (warp ballot into a per-warp list) and run the closest-point search
-    // 32 at a time, so that its lanes are all busy.  Keys are minima, so the
-    // order of the atomics does not matter.
-    __shared__ int queue[4][64];
-    int* qw = queue[(threadIdx.x >> 5) & 3];
+    __syncwarp();
     const unsigned below = (1u << lane) - 1u;
-    int qn = 0;  // warp-uniform queue length (< 32 between rounds)
-    for (int base = 0; base < total; base += 32) {
-        const int i = base + lane;
-        bool pass = false;
-        if (i < total) {
-            int x, y, z;
-            voxel(i, x, y, z);
-            const V3 dcen = cell_world(a.fp, x, y, z) - cen;
-            pass = dot(dcen, dcen) <= reach2;
+    const float quantum = cs * (1.0f / 65536.0f);
+    const int64_t plane = (int64_t)a.bx * a.by;
+    int cn = 0, qn = 0;  // warp-uniform lengths of the column list (< 16 between rounds) and the queue (< 32)
+    auto evaluate = [&](const int4 v) {
+        const RasterTri& r = w.tri[v.w];
+        const float dist = closest_distance(cell_world(a.fp, v.x, v.y, v.z), v3(r.vert[0], r.vert[1], r.vert[2]),
+                                            v3(r.vert[3], r.vert[4], r.vert[5]), v3(r.vert[6], r.vert[7], r.vert[8])) /
+                           cs;
+        const float bin = roundf(dist * 65536.0f);
+        const uint32_t ub = bin >= 4294967295.0f ? 0xFFFFFFFFu : (uint32_t)bin;
+        atomicMin(a.b.keys + ((int64_t)(v.x - ox) + (int64_t)a.bx * (v.y - oy) + plane * (v.z - oz)),
+                  (unsigned long long)ub << 32 | r.id);
+    };
+    // the first `take` (at most 16) listed columns, two lanes each
+    auto walk = [&](int take) {
+        const int e = lane >> 1, half = lane & 1;
+        const int4 c = w.column[e < take ? e : 0];
+        const float2 d = w.offset[e < take ? e : 0];
+        const int t = (uint32_t)c.w >> 28, n = e < take ? c.w & 0x0FFFFFFF : 0;
+        const RasterTri& r = w.tri[t];
+        const float rho2 = d.x * d.x + d.y * d.y, hxy = r.nrm[0] * d.x + r.nrm[1] * d.y, nz = r.nrm[2], cz_ = r.cen[2];
+        const float reach2 = r.reach2, thick = r.thick, disc = r.disc, slack = r.slack;
+        // the distance bins: the keys' high words
+        const uint32_t* bins = (const uint32_t*)(a.b.keys + ((int64_t)(c.x - ox) + (int64_t)a.bx * (c.y - oy) +
+                                                            plane * (c.z - oz))) + 1;
+        for (int k = half; __any_sync(0xffffffffu, k < n); k += 8) {
+            uint32_t bin[4];
+            float dz[4];
+            bool in[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = k + 2 * j;
+                dz[j] = (a.fp.origin[2] + ((float)(c.z + i) + 0.5f) * cs) - cz_;
+                in[j] = i < n && rho2 + dz[j] * dz[j] <= reach2;
+                bin[j] = in[j] ? __ldcg(bins + 2 * plane * i) : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float h = __fmaf_rn(nz, dz[j], hxy);
+                const float hh = fmaxf(fabsf(h) - thick, 0.0f);
+                const float ub = __fmaf_rn((float)bin[j], quantum, slack);
+                const float gap = __fmaf_rn(ub, ub, -hh * hh);
+                const float lat2 = __fmaf_rn(dz[j], dz[j], rho2) - h * h;
+                const float lim = disc + approx_sqrt(fmaxf(gap, 0.0f));
+                const bool keep = in[j] && gap >= 0.0f && lat2 <= lim * lim * 1.0002f;
+                const unsigned m = __ballot_sync(0xffffffffu, keep);
+                if (m == 0) continue;
+                if (keep) w.queue[qn + __popc(m & below)] = make_int4(c.x, c.y, c.z + k + 2 * j, t);
+                qn += __popc(m);
+                __syncwarp();
+                if (qn >= 32) {
+                    const int4 mine = w.queue[lane];
+                    __syncwarp();
+                    if (lane < qn - 32) w.queue[lane] = w.queue[lane + 32];
+                    __syncwarp();
+                    qn -= 32;
+                    evaluate(mine);
+                }
+            }
         }
-        const unsigned m = __ballot_sync(0xffffffffu, pass);
-        if (pass) qw[qn + __popc(m & below)] = i;
-        qn += __popc(m);
-        __syncwarp();
-        if (qn >= 32) {
-            const int mine = qw[lane];
+    };
+    for (int t = 0; t < count; ++t) {
+        const RasterTri& r = w.tri[t];
+        const int ex = r.ext[0], ey = r.ext[1], ez = r.ext[2];
+        if (ex <= 0 || ey <= 0 || ez <= 0) continue;
+        const int lx = r.lo[0], ly = r.lo[1], lz = r.lo[2], columns = ex * ey;
+        const float inv_ex = 1.0f / (float)ex;
+        // cell coordinate of the centroid along z, and what its rounding may be off
+        const float zc = (r.cen[2] - a.fp.origin[2]) / cs - 0.5f, zslack = 0.01f + r.slack / cs;
+        for (int c0 = 0; c0 < columns; c0 += 32) {
+            const int c = c0 + lane;
+            // column -> (x, y) by reciprocal multiplication (exact for these small extents)
+            const int yi = (int)(((float)c + 0.5f) * inv_ex), xi = c - yi * ex;
+            const V3 w0 = cell_world(a.fp, lx + xi, ly + yi, 0);
+            const float dx = w0.x - r.cen[0], dy = w0.y - r.cen[1];
+            const float rest = r.reach2 - (dx * dx + dy * dy);
+            // a superset of the z that pass the sphere test (decided exactly in the walk)
+            const float reach_z = approx_sqrt(fmaxf(rest, 0.0f)) / cs + zslack;
+            const int za = max((int)ceilf(zc - reach_z), lz), zb = min((int)floorf(zc + reach_z), lz + ez - 1);
+            const bool pass = c < columns && rest >= 0.0f && zb >= za;
+            const unsigned m = __ballot_sync(0xffffffffu, pass);
+            if (m == 0) continue;
+            if (pass) {
+                const int at = cn + __popc(m & below);
+                w.column[at] = make_int4(lx + xi, ly + yi, za, (zb - za + 1) | (int)((unsigned)t << 28));
+                w.offset[at] = make_float2(dx, dy);
+            }
+            cn += __popc(m);
             __syncwarp();
-            if (lane < qn - 32) qw[lane] = qw[lane + 32];
-            __syncwarp();
-            qn -= 32;
-            key_voxel(mine);
+            int done = 0;
+            while (cn - done >= 16) {
+                // (the walk reads the list's first entries)
+                if (done) {
+                    const int4 mc = w.column[lane < 16 ? done + lane : 0];
+                    const float2 md = w.offset[lane < 16 ? done + lane : 0];
+                    __syncwarp();
+                    if (lane < 16) {
+                        w.column[lane] = mc;
+                        w.offset[lane] = md;
+                    }
+                    __syncwarp();
+                }
+                walk(16);
+                done += 16;
+                __syncwarp();
+            }
+            if (done) {
+                const int left = cn - done;
+                const int4 mc = w.column[lane < left ? done + lane : 0];
+                const float2 md = w.offset[lane < left ? done + lane : 0];
+                __syncwarp();
+                if (lane < left) {
+                    w.column[lane] = mc;
+                    w.offset[lane] = md;
+                }
+                __syncwarp();
+                cn = left;
+            }
         }
     }
-    if (lane < qn) key_voxel(qw[lane]);
+    if (cn > 0) walk(cn);
+    __syncwarp();
+    if (lane < qn) evaluate(w.queue[lane]);
 }
 
 __device__ bool resolve_cell(const GeomArgs& a, int has_prev, int x, int y, int z, int64_t bidx);
@@ -962,10 +1107,12 @@ __device__ float mesh_ray_root_group(const GeomArgs& a, int fx, int fy, int fz, 
     if (tb >= a.b.ntris) tb = ta;
     const float h = a.b.half_thickness;
     const uint32_t tri = (gl & 1) ? tb : ta;
+    V3 A, B, C;
+    tri_vertices(a, tri, A, B, C);
     // inside (gv <= 0) at the point of parameter t, for the pair of lanes of one point
     auto inside = [&](float t) {
         V3 s = v3(mixf(fw.x, sw.x, t), mixf(fw.y, sw.y, t), mixf(fw.z, sw.z, t));
-        const float d = tri_distance(a, tri, s);
+        const float d = closest_distance(s, A, B, C);
         const float gv = fminf(d, __shfl_xor_sync(gmask, d, 1)) - h;
         return (__ballot_sync(gmask, gv <= 0.0f) >> gshift) & 0x5555u;  // one bit per point: bit 2 * point
     };
@@ -1236,7 +1383,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const GeomArgs a) 
     if (threadIdx.x == 0) sums[blockIdx.x] = t;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const GeomArgs a, int nseg) {
+// At most 56 registers: beside the staged TRT kernel (17 warps of 80) the fullest
+// quarter of an SM has 3,584 free, two warps of this block; with 72 it waited for
+// that kernel's end (0.65 -> 0.60 ms a step on 512 x 256 x 256 plates).
+__global__ void __maxnreg__(56) k_scan_apply(const GeomArgs a, int nseg) {
     __shared__ uint32_t wtot[kScanThreads / 32];
     const bool ev = blockIdx.y != 0;
     const uint32_t* counts = ev ? a.b.event_counts : a.b.block_counts;
@@ -1836,8 +1986,22 @@ void launch_prepare(int geometry, float dt, const GridDesc& g, const FluidParams
     else k_prepare<<<1, 32, 0, s>>>(a, init, dt, 0.0f);
 }
 
+void launch_mesh_keys(const GridDesc& g, const FluidParams& fp, const BoxDesc& box, const GeomBuffers& gb,
+                      cudaStream_t s) {
+    GeomArgs a = make_geom(g, fp, box, gb, nullptr);
+    dim3 sgrid, sblock;
+    slab_shape(box, sgrid, sblock);
+    k_mesh_prepare<<<(gb.nverts + 255) / 256, 256, 0, s>>>(a);
+    k_mesh_clear<<<sgrid, sblock, 0, s>>>(a);
+    // triangles per warp: kRasterTris, fewer while that leaves the SMs short of warps
+    const unsigned per_warp =
+        (unsigned)std::min<int64_t>(kRasterTris, std::max<int64_t>(1, gb.ntris / (gb.topo_blocks * 16)));
+    const unsigned rblocks = (gb.ntris + 4 * per_warp - 1) / (4 * per_warp);  // four warps a block
+    k_mesh_raster<<<rblocks, 128, 0, s>>>(a, (int)per_warp);
+}
+
 void launch_classify(int geometry, int has_prev, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,
-                     const GeomBuffers& gb, cudaStream_t s, bool lean_raster) {
+                     const GeomBuffers& gb, cudaStream_t s) {
     GeomArgs a = make_geom(g, fp, box, gb, nullptr);
     dim3 grid, block;
     box_shape(box, grid, block);
@@ -1850,11 +2014,6 @@ void launch_classify(int geometry, int has_prev, const GridDesc& g, const FluidP
     } else if (geometry == BFX_GEOMETRY_MESH) {
         dim3 sgrid, sblock;
         slab_shape(box, sgrid, sblock);
-        k_mesh_prepare<<<(gb.nverts + 255) / 256, 256, 0, s>>>(a);
-        k_mesh_clear<<<sgrid, sblock, 0, s>>>(a);
-        const unsigned rblocks = (unsigned)(((int64_t)gb.ntris * 32 + 127) / 128);
-        if (lean_raster) k_mesh_raster<1><<<rblocks, 128, 0, s>>>(a);
-        else k_mesh_raster<0><<<rblocks, 128, 0, s>>>(a);
         k_mesh_resolve<<<sgrid, sblock, 0, s>>>(a, has_prev);
     }
 }

@@ -120,6 +120,7 @@ struct GeomBuffers {
     int joint_count;
     const uint32_t* mesh_tris;
     const uint8_t* mesh_tri_part;
+    const uint4* mesh_order;        // triangles (vertices, id) in the order the raster takes them
     float4* mesh_pos;
     float4* mesh_vel;
     unsigned long long* keys;       // box-local
@@ -161,8 +162,11 @@ struct GeomBuffers {
 
 void launch_prepare(int geometry, float dt, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,
                     const GeomBuffers& gb, int init, cudaStream_t s);
+// Mesh: vertices, their bounds and the raster keys (before launch_classify).
+void launch_mesh_keys(const GridDesc& g, const FluidParams& fp, const BoxDesc& box, const GeomBuffers& gb,
+                      cudaStream_t s);
 void launch_classify(int geometry, int has_prev, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,
-                     const GeomBuffers& gb, cudaStream_t s, bool lean_raster = false);
+                     const GeomBuffers& gb, cudaStream_t s);
 // Cut-link and topology-event lists of the step's geometry (counts, offset
 // scan, emission, link fractions).  Reads only geometry: masks, keys, wall
 // field and mesh.

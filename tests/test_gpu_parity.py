@@ -465,3 +465,28 @@ def test_lattice_faces_match_oracle(faces, extent, geometry):
     wide.advance(5)
     # 5 steps of FP32 arithmetic: below 5 x 20 roundings of values near 1/3
     assert np.max(np.abs(wide.populations() - lat.populations())) < 100 * 2.0 ** -25
+
+
+# --------------------------------------------------------------------------
+# Mesh raster: order and size of the triangles
+# --------------------------------------------------------------------------
+@pytest.mark.parametrize("n_chord,n_span,shuffled", [(1, 1, False), (2, 3, True), (16, 48, True), (24, 64, False)])
+def test_raster_matches_oracle(n_chord, n_span, shuffled):
+    """Coarse, fine and scattered triangles: wall velocity and distance of every cell within two
+    cells of the surface (the winning triangle of each raster key), masks and link fractions."""
+    cfg, rows, body, mesh = cases.flapping_plates(nx=72, ny=64, nz=56, span=17.3, chord=6.1, thickness=2.0,
+                                                  n_chord=n_chord, n_span=n_span, period=300.0, viscosity=0.02,
+                                                  sponge_width=6.0)
+    if shuffled:
+        order = np.random.default_rng(11).permutation(mesh["tris"].shape[0])
+        mesh = dict(mesh, tris=mesh["tris"][order], tri_part=mesh["tri_part"][order])
+    lat, osim = make_pair(cfg, rows, body, mesh)
+    for step in range(3):
+        lat.advance(1)
+        osim.step()
+        assert np.array_equal(lat.mask(), osim.mcur)
+        wall, owall = lat.wall(), osim.wall.reshape(-1, 4)
+        near = np.abs(owall[:, 3]) < 1.9
+        assert near.sum() > 500
+        assert np.array_equal(wall[near], owall[near])
+    assert compare_pops(lat, osim, "populations")[1]
