@@ -534,6 +534,20 @@ __device__ __forceinline__ T* canon_slot(T* A, const Grid& g, int rep_s, int q, 
     return A + (int64_t)q * g.pn + pflat(g, x + cx(q), y + cy(q), z + cz(q));
 }
 
+// Velocity of a taped record (rho, u), in 16-byte loads.
+__device__ __forceinline__ void load_velocity(const float* m, float& ux, float& uy, float& uz) {
+    const float4 v = *(const float4*)m;
+    ux = v.y;
+    uy = v.z;
+    uz = v.w;
+}
+__device__ __forceinline__ void load_velocity(const double* m, double& ux, double& uy, double& uz) {
+    const double2 a = ((const double2*)m)[0], b = ((const double2*)m)[1];
+    ux = a.y;
+    uy = b.x;
+    uz = b.y;
+}
+
 // Fluid cells: reverse streaming through the transposed collision.
 template <class R, int REP_S>
 __global__ void __launch_bounds__(256) k_adj_bulk(const AdjArgs a) {
@@ -551,8 +565,8 @@ __global__ void __launch_bounds__(256) k_adj_bulk(const AdjArgs a) {
         if (REP_S) lam[q] = ((const R*)a.plane[opp(q)])[pid];
         else lam[q] = ((const R*)a.plane[q])[(uint32_t)(pid + (uint32_t)a.doff[q])];
     }
-    const R* m = (const R*)a.moments + 4 * (size_t)gid;
-    const R ux = m[1], uy = m[2], uz = m[3];
+    R ux, uy, uz;
+    load_velocity((const R*)a.moments + 4 * (size_t)gid, ux, uy, uz);
     const FluidParams& fp = a.ga.fp;
     if (fp.has_sponge) {
         const float sp = sponge_factor(g, fp, x, y, z);
@@ -764,36 +778,43 @@ __global__ void __launch_bounds__(128) k_adj_halo(const AdjArgs a, int rep_s, in
     }
 }
 
-// Cover / uncover impulses (the forward k_topology): pass 0 covered, pass 1 uncovered.
+// Cover / uncover impulses (the forward k_topology).  A warp's lanes find the
+// events among its 32 cells, then take each event together, lane q direction q:
+// every slot belongs to one (cell, direction), so no two lanes and no two
+// events touch the same one (a covered cell is solid after the step, an
+// uncovered cell's partners are fluid before and after it).  As two launches
+// with one thread per event: 29 us a step on 256 x 128 x 128; now 10 us.
 template <class R>
-__global__ void __launch_bounds__(256) k_adj_topology(const AdjArgs a, int rep_s, int pass) {
+__global__ void __launch_bounds__(256) k_adj_topology(const AdjArgs a, int rep_s) {
     const GeomArgs& ga = a.ga;
     const Grid& g = ga.g;
     const FluidParams& fp = ga.fp;
-    int x, y, z;
-    int64_t bidx;
     if (block_inactive(ga)) return;
-    if (!box_cell(ga, x, y, z, bidx) || !cell_active(ga, x, y, z)) return;
     if (!fp.accumulate || (fp.interpolated && fp.load_component == 1)) return;
-    const int64_t gid = flat(g, x, y, z);
-    const uint8_t mk = ga.b.mask_next[gid];
+    int x = 0, y = 0, z = 0;
+    int64_t bidx;
+    uint8_t mk = 0;
+    if (box_cell(ga, x, y, z, bidx) && cell_active(ga, x, y, z)) mk = ga.b.mask_next[flat(g, x, y, z)];
+    const bool event = (mk & kCovered) != 0 || ((mk & kUncovered) != 0 && fp.force_mode == 6);
+    const int q = linear_tid() & 31;
     const double s = a.weight * (double)fp.f2p;
     const double* wF = a.obj->force_weight;
     R* A = (R*)a.lam;
-    if (pass == 0 && (mk & kCovered)) {
-        for (int q = 0; q < 19; ++q) {
-            const double c = wF[0] * cx(q) + wF[1] * cy(q) + wF[2] * cz(q);
-            if (c != 0.0) *canon_slot(A, g, rep_s, q, x, y, z) += (R)(s * c);
-        }
-    } else if (pass == 1 && (mk & kUncovered) && fp.force_mode == 6) {
-        for (int q = 1; q < 19; ++q) {
-            const int nx_ = x + cx(q), ny_ = y + cy(q), nz_ = z + cz(q);
+    for (unsigned events = __ballot_sync(0xffffffffu, event); events; events &= events - 1) {
+        const int from = __ffs(events) - 1;
+        const int ex = __shfl_sync(0xffffffffu, x, from), ey = __shfl_sync(0xffffffffu, y, from),
+                  ez = __shfl_sync(0xffffffffu, z, from);
+        const bool covered = (__shfl_sync(0xffffffffu, (int)mk, from) & kCovered) != 0;
+        if (q >= 19) continue;
+        const double c = wF[0] * cx(q) + wF[1] * cy(q) + wF[2] * cz(q);
+        if (covered) {
+            if (c != 0.0) *canon_slot(A, g, rep_s, q, ex, ey, ez) += (R)(s * c);
+        } else if (q > 0 && c != 0.0) {
+            const int nx_ = ex + cx(q), ny_ = ey + cy(q), nz_ = ez + cz(q);
             if (!inside(g, nx_, ny_, nz_)) continue;
             const int64_t nb = flat(g, nx_, ny_, nz_);
             if (!((ga.b.mask_prev[nb] & kPartMask) == 0 && (ga.b.mask_next[nb] & kPartMask) == 0)) continue;
-            const double c = wF[0] * cx(q) + wF[1] * cy(q) + wF[2] * cz(q);
-            if (c == 0.0) continue;
-            *canon_slot(A, g, rep_s, q, x, y, z) -= (R)(s * c);
+            *canon_slot(A, g, rep_s, q, ex, ey, ez) -= (R)(s * c);
             *canon_slot(A, g, rep_s, opp(q), nx_, ny_, nz_) -= (R)(s * c);
         }
     }
@@ -827,16 +848,27 @@ __global__ void __launch_bounds__(256) k_adj_init(const AdjArgs a, int rep_s) {
     write_partials<NP>(grad, a.part_rare);
 }
 
-__global__ void k_adj_reduce(const double* rare, int nrare, const double* links, int nlinks, Objective* obj) {
-    __shared__ double sh[NP][256];
+// One block: fixed-order sums of the block partials (strided per thread, then
+// shuffles, then over the warps).
+constexpr int kAdjReduceThreads = 1024;
+__global__ void __launch_bounds__(kAdjReduceThreads) k_adj_reduce(const double* rare, int nrare, const double* links,
+                                                                  int nlinks, Objective* obj) {
+    __shared__ double sh[NP][kAdjReduceThreads / 32];
     double acc[NP] = {0.0, 0.0, 0.0, 0.0};
     for (int i = threadIdx.x; i < nrare; i += blockDim.x)
         for (int k = 0; k < NP; ++k) acc[k] += rare[NP * i + k];
     for (int i = threadIdx.x; i < nlinks; i += blockDim.x)
         for (int k = 0; k < NP; ++k) acc[k] += links[NP * i + k];
-    block_sum<NP>(acc, sh);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < NP; ++k) obj->grad[k] += acc[k];
+    for (int o = 16; o > 0; o >>= 1)
+        for (int k = 0; k < NP; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < NP; ++k) sh[k][threadIdx.x >> 5] = acc[k];
+    __syncthreads();
+    if (threadIdx.x < NP) {
+        double v = 0.0;
+        for (int w = 0; w < kAdjReduceThreads / 32; ++w) v += sh[threadIdx.x][w];
+        obj->grad[threadIdx.x] += v;
+    }
 }
 
 }  // namespace
@@ -873,9 +905,8 @@ static void adjoint_step_t(int rep_s, const GridDesc& gd, const BoxDesc& box, Ad
     k_adj_links2<R><<<apply_blocks, 256, 0, s>>>(a, rep_s);
     const int64_t halo = a.ga.g.pn - a.ga.g.n;
     k_adj_halo<R><<<(unsigned)((halo + 127) / 128), 128, 0, s>>>(a, rep_s, halo);
-    k_adj_topology<R><<<bgrid, bblock, 0, s>>>(a, rep_s, 0);
-    k_adj_topology<R><<<bgrid, bblock, 0, s>>>(a, rep_s, 1);
-    k_adj_reduce<<<1, 256, 0, s>>>(a.part_rare, (int)(bgrid.x * bgrid.y * bgrid.z), a.part_links, apply_blocks, a.obj);
+    k_adj_topology<R><<<bgrid, bblock, 0, s>>>(a, rep_s);
+    k_adj_reduce<<<1, kAdjReduceThreads, 0, s>>>(a.part_rare, (int)(bgrid.x * bgrid.y * bgrid.z), a.part_links, apply_blocks, a.obj);
 }
 
 static AdjArgs adjoint_args(int storage, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,
@@ -919,7 +950,7 @@ void launch_adjoint_init(int storage, int rep_s, const GridDesc& g, const FluidP
     box_shape(box, bgrid, bblock);
     if (storage == BFX_STORAGE_F64) k_adj_init<double><<<bgrid, bblock, 0, s>>>(a, rep_s);
     else k_adj_init<float><<<bgrid, bblock, 0, s>>>(a, rep_s);
-    k_adj_reduce<<<1, 256, 0, s>>>(a.part_rare, (int)(bgrid.x * bgrid.y * bgrid.z), a.part_links, 0, a.obj);
+    k_adj_reduce<<<1, kAdjReduceThreads, 0, s>>>(a.part_rare, (int)(bgrid.x * bgrid.y * bgrid.z), a.part_links, 0, a.obj);
 }
 
 }  // namespace bfx

@@ -159,6 +159,9 @@ struct bfx_sim {
     uint64_t pipe_launches[2] = {0, 0};
     // side stream of the next step's geometry build, with its fork / join events
     cudaStream_t side = nullptr;
+    // the adjoint's wing-frame tangent (one thread, 50 us) beside that build
+    cudaStream_t tangent = nullptr;
+    cudaEvent_t tangent_ev = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr, lists_ev = nullptr;
     cudaEvent_t halo_fork_ev = nullptr, halo_join_ev = nullptr;
     // topology record / replay test hook (bfx_test_replay_topology): 0 off,
@@ -389,6 +392,26 @@ void encode_links(bfx_sim* s, uint8_t* mprev, uint8_t* mnext) {
     if (s->moving()) encode_topology(s, mprev, mnext);
 }
 
+// What a taped step records beside the fluid kernel's moments: the wing-frame
+// tangent of the step the state is about to take, the link tangents, and the
+// masks and keys.
+void encode_frame_tangent(bfx_sim* s, uint8_t* mprev, uint8_t* mnext, const TapeSlot& tape, cudaStream_t st) {
+    launch_frame_tangent(geom_buffers(s, mprev, mnext), s->cfg.time_step, 0, tape.frames, st);
+    s->launches += 1;
+}
+void encode_link_tangent(bfx_sim* s, uint8_t* mprev, uint8_t* mnext, const TapeSlot& tape, cudaStream_t st) {
+    GeomBuffers gb = geom_buffers(s, mprev, mnext);
+    gb.frames = tape.frames;
+    launch_link_tangent(s->cfg.link_rule, s->fp.interpolated, s->g, s->fp, s->box, gb, tape.link_tangent, st);
+    s->launches += 1;
+}
+void encode_geometry_tape(bfx_sim* s, uint8_t* mprev, uint8_t* mnext, const TapeSlot& tape, cudaStream_t st) {
+    cudaMemcpyAsync(tape.mask_next, mnext, (size_t)s->g.n, cudaMemcpyDeviceToDevice, st);
+    cudaMemcpyAsync(tape.mask_prev, mprev, (size_t)s->g.n, cudaMemcpyDeviceToDevice, st);
+    cudaMemcpyAsync(tape.keys, s->keys, (size_t)s->box.cells * sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
+                    st);
+}
+
 void timing_begin(bfx_sim* s) {
     if (!s->timing) return;
     if (s->ev_used >= s->ev_start.size()) {
@@ -421,10 +444,12 @@ void timing_collect(bfx_sim* s) {
 // and link tangents, the link values, masks, keys, state and pre-collision moments.
 // geometry_ready: this step's geometry was built by the previous step's
 // prefetch.  prefetch_next: build the next step's geometry on the side stream
-// while this step's fluid kernel runs (can_pipeline; no capture, tape or ledger).
+// while this step's fluid kernel runs (can_pipeline; no capture or ledger); a
+// taped step also takes the next step's tape slot and leaves its wing-frame and
+// link tangents there.
 void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint64_t sample_index,
                  const TapeSlot* tape = nullptr, double* ledger_in = nullptr, bool geometry_ready = false,
-                 bool prefetch_next = false) {
+                 bool prefetch_next = false, const TapeSlot* next_tape = nullptr) {
     s->hstate_fresh = false;
     uint8_t* mprev = s->mask[s->cur];
     uint8_t* mnext = s->moving() ? s->mask[s->cur ^ 1] : s->mask[s->cur];
@@ -451,20 +476,11 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
             else cudaMemcpyAsync(mnext, rec, (size_t)s->g.n, cudaMemcpyDeviceToDevice, s->stream);
         }
     }
-    if (tape) {
-        launch_frame_tangent(geom_buffers(s, mprev, mnext), s->cfg.time_step, 0, tape->frames, s->stream);
-        s->launches += 1;
-    }
+    if (tape && !geometry_ready) encode_frame_tangent(s, mprev, mnext, *tape, s->stream);
     // geometry_ready: the previous step built this step's cut-link and event
     // lists with its geometry and ran its topology impulses
     if (s->geometry() && s->moving() && !geometry_ready) encode_links(s, mprev, mnext);
-    if (tape) {
-        GeomBuffers gb = geom_buffers(s, mprev, mnext);
-        gb.frames = tape->frames;
-        launch_link_tangent(s->cfg.link_rule, s->fp.interpolated, s->g, s->fp, s->box, gb, tape->link_tangent,
-                            s->stream);
-        s->launches += 1;
-    }
+    if (tape && !geometry_ready) encode_link_tangent(s, mprev, mnext, *tape, s->stream);
     if (ledger_in) {
         // the ledger's pre-step pass: geometry built, no population written yet
         launch_ledger_in(s->cfg.storage, s->rep_s, s->g, s->fp, fb, s->geometry() ? mprev : nullptr,
@@ -492,7 +508,7 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
                            finish_fused ? &fin : nullptr, s->stream);
         s->launches += 1;
     }
-    const bool pipelined = prefetch_next && capture == 0 && !tape && !ledger_in && can_pipeline(s);
+    const bool pipelined = prefetch_next && capture == 0 && !ledger_in && can_pipeline(s);
     const int box[3] = {s->box.sx, s->box.sy, s->box.sz};
     if (pipelined) {
         // The solid / uncovered cells right after the link kernel, beside the
@@ -503,13 +519,17 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     }
     if (halo_side) cudaStreamWaitEvent(s->stream, s->halo_join_ev, 0);
     if (tape) {
+        // the state between the loads and the body update, then the update
+        // (the next step's pose reads it)
         cudaMemcpyAsync(tape->state, s->dstate, sizeof(DeviceState), cudaMemcpyDeviceToDevice, s->stream);
-        cudaMemcpyAsync(tape->mask_next, mnext, (size_t)s->g.n, cudaMemcpyDeviceToDevice, s->stream);
-        cudaMemcpyAsync(tape->mask_prev, mprev, (size_t)s->g.n, cudaMemcpyDeviceToDevice, s->stream);
-        cudaMemcpyAsync(tape->keys, s->keys, (size_t)s->box.cells * sizeof(unsigned long long),
-                        cudaMemcpyDeviceToDevice, s->stream);
+        launch_integrate(s->g, s->fp, geom_buffers(s, mprev, mnext), fin.gravity[0], fin.gravity[1], fin.gravity[2],
+                         fin.substeps, fin.free_flight, s->stream);
+        s->launches += 1;
         fb.tape = tape->moments;
         capture = 2;
+        // the masks and keys beside the fluid kernel when the next step's
+        // geometry, which rewrites them, follows on the side stream
+        if (!pipelined) encode_geometry_tape(s, mprev, mnext, *tape, s->stream);
     }
     if (pipelined) {
         // Beside the fluid kernel, on the side stream: the next step's
@@ -523,12 +543,20 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
         if (early) encode_pose(s, 0, mnext, mprev, s->stream);
         cudaEventRecord(s->fork_ev, s->stream);
         cudaStreamWaitEvent(s->side, s->fork_ev, 0);
+        if (tape) encode_geometry_tape(s, mprev, mnext, *tape, s->side);
         if (!early) encode_pose(s, 0, mnext, mprev, s->side);
         encode_classify(s, 0, mnext, mprev, s->side);
         if (s->geometry()) encode_link_build(s, mnext, mprev, s->side, s->lists_ev);
         else cudaEventRecord(s->lists_ev, s->side);
+        if (next_tape) {
+            cudaStreamWaitEvent(s->tangent, s->fork_ev, 0);
+            encode_frame_tangent(s, mnext, mprev, *next_tape, s->tangent);
+            cudaEventRecord(s->tangent_ev, s->tangent);
+            cudaStreamWaitEvent(s->side, s->tangent_ev, 0);
+            encode_link_tangent(s, mnext, mprev, *next_tape, s->side);
+        }
         cudaEventRecord(s->join_ev, s->side);
-        launch_bulk_fluid(s->cfg.storage, s->cfg.collision, s->rep_s, s->g, s->fp, fb, box, s->stream);
+        launch_bulk_fluid(s->cfg.storage, s->cfg.collision, s->rep_s, s->g, s->fp, fb, capture, box, s->stream);
     } else {
         timing_begin(s);
         launch_bulk(s->cfg.storage, s->cfg.collision, s->rep_s, s->g, s->fp, fb, capture,
@@ -537,7 +565,7 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     }
     s->launches += pipelined ? 2 : launch_bulk_count(s->cfg.storage, s->cfg.collision, capture, s->tma_ok, s->geometry());
     GeomBuffers gb = geom_buffers(s, mprev, mnext);
-    if (!finish_fused && !counted) {
+    if (!finish_fused && !counted && !tape) {
         launch_integrate(s->g, s->fp, gb, fin.gravity[0], fin.gravity[1], fin.gravity[2], fin.substeps,
                          fin.free_flight, s->stream);
         s->launches += 1;
@@ -600,6 +628,30 @@ int run_steps_graph(bfx_sim* s, int nsteps, bool pipelined = false) {
     return BFX_OK;
 }
 int run_pair_graph(bfx_sim* s) { return run_steps_graph(s, 2); }
+
+// `count` steps without capture, samples or tape.  Pipelined where possible:
+// every step but the last builds the next step's geometry beside its own fluid
+// kernel; the first builds its own, pairs replay a graph while a step remains
+// after them, the last one or two run directly.
+int run_plain_steps(bfx_sim* s, uint64_t count) {
+    uint64_t k = 0;
+    if (s->graphs_enabled && !s->timing && !s->topo_mode && can_pipeline(s) && count > 1) {
+        encode_step(s, 0, nullptr, 0, nullptr, nullptr, false, true);
+        for (k = 1; k + 2 < count; k += 2) {
+            const int rc = run_steps_graph(s, 2, true);
+            if (rc != BFX_OK) return rc;
+        }
+        for (; k < count; ++k) encode_step(s, 0, nullptr, 0, nullptr, nullptr, true, k + 1 < count);
+        return BFX_OK;
+    }
+    if (s->graphs_enabled && !s->timing)
+        for (; k + 1 < count; k += 2) {
+            const int rc = run_pair_graph(s);
+            if (rc != BFX_OK) return rc;
+        }
+    for (; k < count; ++k) encode_step(s, 0, nullptr, 0);
+    return BFX_OK;
+}
 
 int sync_check(bfx_sim* s, const char* what) {
     cudaError_t e = cudaStreamSynchronize(s->stream);
@@ -830,6 +882,8 @@ void bfx_destroy(bfx_sim* s) {
     if (s->lists_ev) cudaEventDestroy(s->lists_ev);
     if (s->halo_fork_ev) cudaEventDestroy(s->halo_fork_ev);
     if (s->halo_join_ev) cudaEventDestroy(s->halo_join_ev);
+    if (s->tangent_ev) cudaEventDestroy(s->tangent_ev);
+    if (s->tangent) cudaStreamDestroy(s->tangent);
     if (s->side) cudaStreamDestroy(s->side);
     if (s->hstate) cudaFreeHost(s->hstate);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -876,6 +930,8 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
     // side stream for the pipelined geometry build (optional: without it the
     // steps run in order on the main stream)
     if (cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, side_priority) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&s->tangent, cudaStreamNonBlocking, side_priority) != cudaSuccess ||
+        cudaEventCreateWithFlags(&s->tangent_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->join_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->lists_ev, cudaEventDisableTiming) != cudaSuccess ||
@@ -2051,13 +2107,8 @@ int bfx_adjoint(bfx_sim* s, uint64_t steps, const bfx_adjoint_objective* objecti
     for (uint64_t seg = 0; seg < nseg; ++seg) {
         snapshot(seg);
         const uint64_t len = std::min<uint64_t>(K, steps - seg * K);
-        uint64_t k = 0;
-        if (s->graphs_enabled && !s->timing)
-            for (; k + 1 < len; k += 2) {
-                rc = run_pair_graph(s);
-                if (rc != BFX_OK) return rc;
-            }
-        for (; k < len; ++k) encode_step(s, 0, nullptr, 0);
+        rc = run_plain_steps(s, len);
+        if (rc != BFX_OK) return rc;
     }
     snapshot(nseg);
     cudaEventRecord(ev[1], s->stream);
@@ -2127,10 +2178,12 @@ int bfx_adjoint(bfx_sim* s, uint64_t steps, const bfx_adjoint_objective* objecti
         // the tape holds link_slots links per step: cap the link list there (the
         // recomputation reproduces the forward pass, whose largest count it is)
         s->link_capacity = (uint32_t)link_slots;
+        const bool pipelined = can_pipeline(s) && !s->timing;
         for (uint64_t j = 0; j < len; ++j) {
             reps[j] = s->rep_s;
-            TapeSlot t = slot(j);
-            encode_step(s, 0, nullptr, 0, &t);
+            const TapeSlot t = slot(j), next = slot(j + 1 < len ? j + 1 : j);
+            const bool more = pipelined && j + 1 < len;
+            encode_step(s, 0, nullptr, 0, &t, nullptr, pipelined && j > 0, more, more ? &next : nullptr);
         }
         s->link_capacity = saved_capacity;
         for (uint64_t j = len; j-- > 0;) {
@@ -2148,7 +2201,7 @@ int bfx_adjoint(bfx_sim* s, uint64_t steps, const bfx_adjoint_objective* objecti
             GeomBuffers gb = geom_buffers(s, s->mask[0], s->mask[1]);
             gb.link_capacity = (uint32_t)link_slots;  // the tape slot's size
             launch_adjoint_step(s->cfg.storage, reps[j], s->g, s->fp, s->box, gb, tape, w, weight, s->stream);
-            s->launches += 9;
+            s->launches += 7;
         }
         cudaError_t le = cudaGetLastError();
         if (le != cudaSuccess) return cuda_fail(s, le, "adjoint launch");

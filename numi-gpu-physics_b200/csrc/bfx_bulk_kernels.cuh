@@ -361,6 +361,15 @@ __device__ __forceinline__ void moments(const R (&f)[19], R& rho, R& ux, R& uy, 
 #endif
 }
 
+// One taped record (rho, u), in 16-byte stores.
+__device__ __forceinline__ void store_moments(float* t, float rho, float ux, float uy, float uz) {
+    *(float4*)t = make_float4(rho, ux, uy, uz);
+}
+__device__ __forceinline__ void store_moments(double* t, double rho, double ux, double uy, double uz) {
+    ((double2*)t)[0] = make_double2(rho, ux);
+    ((double2*)t)[1] = make_double2(uy, uz);
+}
+
 // Sponge relaxation toward the far field, captured fields, limiter statistics.
 template <class S, int COLL>
 __device__ __forceinline__ void finish_cell(const BulkArgs& a, uint32_t gid, int x, int y, int z, bool capture,
@@ -486,11 +495,7 @@ __global__ void __launch_bounds__(256, sizeof(typename S::R) == 8 ? 1 : (COLL ==
         moments<R>(f, rho, ux, uy, uz);
         if (CAPTURE == 2) {
             // adjoint tape: the collision Jacobian depends on the pre-collision moments only
-            R* t = (R*)a.tape + 4 * (size_t)gid;
-            t[0] = rho;
-            t[1] = ux;
-            t[2] = uy;
-            t[3] = uz;
+            store_moments((R*)a.tape + 4 * (size_t)gid, rho, ux, uy, uz);
         }
         collide<R, COLL>(f, rho, ux, uy, uz, (R)a.fp.omega_p, (R)a.fp.omega_m, post, activation, restriction);
     }

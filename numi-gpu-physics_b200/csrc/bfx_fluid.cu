@@ -463,11 +463,11 @@ void launch_bulk_rare(int storage, int collision, int rep_s, const GridDesc& g, 
     else exact::rare_s<StoreF32>(a, collision, rep_s, s);
 }
 void launch_bulk_fluid(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
-                       const FluidBuffers& b, const int* box, cudaStream_t s) {
-    BulkArgs a = make_bulk_args(g, fp, b, 0, storage);
+                       const FluidBuffers& b, int capture, const int* box, cudaStream_t s) {
+    BulkArgs a = make_bulk_args(g, fp, b, capture, storage);
     for (int k = 0; k < 3; ++k) a.box[k] = box[k];
     a.skip_rare = 1;
-    if (use_staged(storage, collision, 0, b.tmap != nullptr))
+    if (use_staged(storage, collision, capture, b.tmap != nullptr))
         launch_stream_fast(storage, collision, rep_s, g, &a, (const CUtensorMap*)b.tmap, b.sm_count, s);
     else if (contracted(storage, fp)) launch_bulk_fast(storage, collision, rep_s, g, a, s);
     else if (storage == BFX_STORAGE_F64) exact::bulk_s<StoreF64>(a, g, collision, rep_s, s);

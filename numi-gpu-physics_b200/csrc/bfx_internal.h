@@ -66,7 +66,7 @@ void launch_halo_yz(int storage, int rep_s, const GridDesc& g, const FluidParams
 void launch_bulk_rare(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
                       const FluidBuffers& b, const int* box, cudaStream_t s);
 void launch_bulk_fluid(int storage, int collision, int rep_s, const GridDesc& g, const FluidParams& fp,
-                        const FluidBuffers& b, const int* box, cudaStream_t s);
+                       const FluidBuffers& b, int capture, const int* box, cudaStream_t s);
 // Block counts per segment of the two-level link-offset scan (bfx_geometry.cu).
 constexpr int kScanSegment = 8192;
 
