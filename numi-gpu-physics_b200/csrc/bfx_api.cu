@@ -1042,7 +1042,7 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
         s->hstate = nullptr;  // pageable copies instead
     }
     BFX_ALLOC(s->dobjective, sizeof(Objective));
-    s->mm_blocks = 4 * s->sm_count;
+    s->mm_blocks = 2 * s->sm_count;  // the resident blocks of k_mass_momentum
     BFX_ALLOC(s->mm_partials, (size_t)s->mm_blocks * 4 * sizeof(double));
     BFX_ALLOC(s->mm_result, 4 * sizeof(double));
 
