@@ -125,7 +125,8 @@ struct bfx_sim {
     int mm_blocks = 0;
     float* scratch_f32 = nullptr;  // canonical read-out staging (lazily)
     FaceEquilibria faces{};        // far-field / velocity face values of the fused kernel,
-    bool inline_faces = false;     // which takes the faces itself (bulk_inline_faces)
+    int inline_faces = 0;          // and which of them it takes itself (bulk_inline_faces)
+    bool solid_clear = false;      // static geometry that stays clear of every face
     int face_ready = 0;            // faces the staged kernel takes from face_dev without their fill: 0, 2 (x) or 6
     float face_dev[6 * 19] = {};   // their values (stored deviations, host copy)
     bfx_run_sample* dsamples = nullptr;
@@ -235,6 +236,7 @@ FluidBuffers fluid_buffers(bfx_sim* s, uint8_t* mask) {
     b.face_dev = s->face_ready ? s->face_dev : nullptr;
     b.face_count = s->face_ready;
     b.faces = s->inline_faces ? &s->faces : nullptr;
+    b.inline_faces = s->inline_faces;
     b.count_step = 0;
     return b;
 }
@@ -349,9 +351,12 @@ bool x_faces_constant(const bfx_config& c) { return faces_constant(c, 0, 1); }
 // cell is never solid), and reads nothing they write.  A periodic face's fill
 // copies real cells that a link may overwrite, an outflow face's copies its
 // interior neighbour, and a link whose solid source is a periodic image writes
-// a halo slot: those keep the fill first on the main stream.
+// a halo slot: those keep the fill first on the main stream, unless the
+// geometry is static and clear of the faces (then no link's source is an image,
+// and an outflow copy reads fluid cells' slots, which no link writes).
 bool halo_beside_links(const bfx_sim* s) {
-    return s->moving() && s->side != nullptr && faces_constant(s->cfg) && !s->inline_faces && s->face_ready != 6;
+    if (s->side == nullptr || s->inline_faces == 1 || s->face_ready == 6) return false;
+    return s->moving() ? faces_constant(s->cfg) : s->solid_clear;
 }
 // Without geometry and without a body update the end of a step is its counter
 // alone: the fused kernel counts it (not BF16, whose stochastic stores read
@@ -362,10 +367,10 @@ bool step_counted_by_bulk(const bfx_sim* s) {
 
 // The halo fill the step's fused kernel needs, on one stream: none where it
 // takes the faces itself, the y / z faces for the staged kernel with x-face
-// values, or every face.
+// values or FP32 / FP64 with inline x faces, or every face.
 void encode_halo(bfx_sim* s, const FluidBuffers& fb, bool staged, cudaStream_t st) {
-    const bool yz_only = staged && s->face_ready != 0;
-    if (s->inline_faces || (staged && s->face_ready == 6)) return;
+    const bool yz_only = staged ? s->face_ready != 0 : s->inline_faces == 2;
+    if (s->inline_faces == 1 || (staged && s->face_ready == 6)) return;
     if (yz_only) launch_halo_yz(s->cfg.storage, s->rep_s, s->g, s->fp, fb, st);
     else launch_halo(s->cfg.storage, s->rep_s, s->g, s->fp, fb, st);
     s->launches += 1;
@@ -1068,6 +1073,13 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
         // geometry box
         float r = geometry_radius(&c, &s->bird, mesh);
         int half = (int)std::ceil(r / c.cell_size) + 4;
+        // r already holds two cells beyond the geometry
+        s->solid_clear = c.static_geometry != 0;
+        for (int k = 0; k < 3; ++k) {
+            const double at = (hs.body[k] - c.origin[k]) / c.cell_size, reach = r / c.cell_size;
+            const int dim = k == 0 ? g.nx : (k == 1 ? g.ny : g.nz);
+            s->solid_clear = s->solid_clear && at - reach > 1.0 && at + reach < dim - 1.0;
+        }
         int ext = 2 * half + 2;
         s->box.sx = std::min(ext, g.nx);
         s->box.sy = std::min(ext, g.ny);

@@ -25,7 +25,7 @@ struct BulkArgs {
     // 2: every face (no fill at all)
     int face_values;
     float face_dev[6][19];
-    int inline_faces;       // k_bulk takes the faces itself (load_cell_edge), no halo fill
+    int inline_faces;       // k_bulk takes faces itself: 0 none, 1 every face (load_cell_edge), 2 the x faces
     int skip_rare;          // k_bulk leaves solid / newly uncovered cells to k_rare (pipelined step)
     int count_step;         // the fused kernel also counts the step (no end-of-step kernel)
     FaceEquilibria faces;

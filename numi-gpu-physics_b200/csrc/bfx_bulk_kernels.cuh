@@ -303,6 +303,24 @@ __device__ __forceinline__ void load_cell_edge(const BulkArgs& a, int x, int y, 
     }
 }
 
+// Far-field / velocity x faces of a cell loaded from the slots (FACES 2): the
+// values k_halo would have written there, also for sources outside in y or z
+// (exit_face takes the x face first).
+template <class R>
+__device__ __forceinline__ void x_faces(const BulkArgs& a, int x, R (&f)[19]) {
+    const auto face = [&](int k, int q) { return sizeof(R) == 8 ? (R)a.faces.d[k][q] : (R)a.faces.f[k][q]; };
+    if (x == 0) {
+#pragma unroll
+        for (int q = 1; q < 19; ++q)
+            if (cx(q) > 0) f[q] = face(0, q);
+    }
+    if (x == a.g.nx - 1) {
+#pragma unroll
+        for (int q = 1; q < 19; ++q)
+            if (cx(q) < 0) f[q] = face(1, q);
+    }
+}
+
 template <class S, int REP_S>
 __device__ __forceinline__ void store_cell(const BulkArgs& a, uint32_t pid, const typename S::R (&post)[19]) {
     using T = typename S::T;
@@ -446,10 +464,10 @@ __device__ __forceinline__ void rare_cell(const BulkArgs& a, uint32_t gid, int x
 
 // ---------------------------------------------------------------------------
 // The fused kernel: every cell of the lattice; solid and newly uncovered
-// cells (flagged in the mask) take rare_cell.  FACES 1 (FP32 and FP64 on small
-// lattices, bulk_inline_faces) also takes the lattice faces, so no halo fill
-// precedes the kernel: its launch was a third of the step on a 64^3 periodic
-// lattice.
+// cells (flagged in the mask) take rare_cell.  FACES (FP32 and FP64,
+// bulk_inline_faces): 1 also takes every lattice face, so no halo fill precedes
+// the kernel (its launch was a third of the step on a 64^3 periodic lattice); 2
+// takes the x faces.
 // ---------------------------------------------------------------------------
 template <class S, int REP_S, int COLL, int CAPTURE, int FACES>
 __global__ void __launch_bounds__(256, sizeof(typename S::R) == 8 ? 1 : (COLL == BFX_COLLISION_TRT_LIMITER ? 2 : 4))
@@ -472,12 +490,13 @@ __global__ void __launch_bounds__(256, sizeof(typename S::R) == 8 ? 1 : (COLL ==
         }
     }
     R f[19];
-    if constexpr (FACES) {
+    if constexpr (FACES == 1) {
         const bool edge = x == 0 || x == a.g.nx - 1 || y == 0 || y == a.g.ny - 1 || z == 0 || z == a.g.nz - 1;
         if (__any_sync(__activemask(), edge)) load_cell_edge<S, REP_S>(a, x, y, z, pid, f);
         else load_cell<S, REP_S>(a, pid, f);
     } else {
         load_cell<S, REP_S>(a, pid, f);
+        if constexpr (FACES == 2) x_faces<R>(a, x, f);
     }
     R post[19];
     float activation = 0.0f, restriction = 0.0f;
@@ -558,27 +577,24 @@ static void rare_s(const BulkArgs& a, int collision, int rep_s, cudaStream_t s) 
     }
 }
 
+template <class S, int REP, int COLL, int FACES>
+static void bulk_f(const BulkArgs& a, const dim3& grid, const dim3& block, cudaStream_t s) {
+    if (a.capture == 1) k_bulk<S, REP, COLL, 1, FACES><<<grid, block, 0, s>>>(a);
+#ifndef BFX_CONTRACTED
+    else if (a.capture == 2 && COLL == BFX_COLLISION_TRT)
+        k_bulk<S, REP, BFX_COLLISION_TRT, 2, FACES><<<grid, block, 0, s>>>(a);
+#endif
+    else k_bulk<S, REP, COLL, 0, FACES><<<grid, block, 0, s>>>(a);
+}
 template <class S, int REP, int COLL>
 static void bulk_t(const BulkArgs& a, const GridDesc& g, cudaStream_t s) {
     dim3 grid, block;
     cell_launch_shape(g, grid, block);
     if constexpr (sizeof(typename S::T) >= 4) {
-        if (a.inline_faces) {
-            if (a.capture == 1) k_bulk<S, REP, COLL, 1, 1><<<grid, block, 0, s>>>(a);
-#ifndef BFX_CONTRACTED
-            else if (a.capture == 2 && COLL == BFX_COLLISION_TRT)
-                k_bulk<S, REP, BFX_COLLISION_TRT, 2, 1><<<grid, block, 0, s>>>(a);
-#endif
-            else k_bulk<S, REP, COLL, 0, 1><<<grid, block, 0, s>>>(a);
-            return;
-        }
+        if (a.inline_faces == 1) return bulk_f<S, REP, COLL, 1>(a, grid, block, s);
+        if (a.inline_faces == 2) return bulk_f<S, REP, COLL, 2>(a, grid, block, s);
     }
-    if (a.capture == 1) k_bulk<S, REP, COLL, 1, 0><<<grid, block, 0, s>>>(a);
-#ifndef BFX_CONTRACTED
-    else if (a.capture == 2 && COLL == BFX_COLLISION_TRT)
-        k_bulk<S, REP, BFX_COLLISION_TRT, 2, 0><<<grid, block, 0, s>>>(a);
-#endif
-    else k_bulk<S, REP, COLL, 0, 0><<<grid, block, 0, s>>>(a);
+    bulk_f<S, REP, COLL, 0>(a, grid, block, s);
 }
 
 template <class S>

@@ -317,11 +317,15 @@ FaceEquilibria make_face_equilibria(const FluidParams& fp) {
     return e;
 }
 
-bool bulk_inline_faces(int storage, const GridDesc& g, const FluidParams& fp, bool geometry) {
-    if (storage != BFX_STORAGE_F32 && storage != BFX_STORAGE_F64) return false;
-    for (int f = 0; f < 6; ++f)
-        if (fp.face_bc[f] == BFX_BC_OUTFLOW || (fp.face_bc[f] == BFX_BC_PERIODIC && geometry)) return false;
-    return g.n <= kInlineFaceCells;
+int bulk_inline_faces(int storage, const GridDesc& g, const FluidParams& fp, bool geometry) {
+    if (storage != BFX_STORAGE_F32 && storage != BFX_STORAGE_F64) return 0;
+    bool every = g.n <= kInlineFaceCells, x_values = true;
+    for (int f = 0; f < 6; ++f) {
+        const bool value = fp.face_bc[f] == BFX_BC_FARFIELD || fp.face_bc[f] == BFX_BC_VELOCITY;
+        every = every && (value || (fp.face_bc[f] == BFX_BC_PERIODIC && !geometry));
+        if (f < 2) x_values = x_values && value;
+    }
+    return every ? 1 : (x_values ? 2 : 0);
 }
 
 Grid device_grid(const GridDesc& gd) {
@@ -359,7 +363,7 @@ BulkArgs make_bulk_args(const GridDesc& gd, const FluidParams& fp, const FluidBu
     for (int f = 0; f < 6; ++f)
         for (int q = 0; q < 19; ++q) a.face_dev[f][q] = b.face_dev ? b.face_dev[19 * f + q] : 0.0f;
     if (b.faces) a.faces = *b.faces;
-    a.inline_faces = b.faces ? 1 : 0;
+    a.inline_faces = b.faces ? b.inline_faces : 0;
     a.count_step = b.count_step;
     a.skip_rare = 0;
     a.pops = b.pops;

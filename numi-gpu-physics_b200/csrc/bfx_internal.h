@@ -36,7 +36,8 @@ struct FluidBuffers {
     void* tape;             // pre-collision (rho, u) per cell when the step is taped (capture == 2)
     const void* tmap;       // CUtensorMap of the population array for the staged kernel (null: k_bulk)
     int sm_count;
-    const FaceEquilibria* faces;  // host copy; null: the halo fill covers the faces
+    const FaceEquilibria* faces;  // host copy; null: the halo fill covers every face
+    int inline_faces;       // faces k_bulk takes from them: 1 every face, 2 the x faces
     int count_step;         // the fused kernel counts the step (no geometry, no body update)
     const float* face_dev;  // host copy of the face values [6][19] for the staged kernel (null: the halo
                             // fill covers every face)
@@ -78,17 +79,20 @@ void launch_flow_diagnostics(const float4* velocity, const uint8_t* mask, int nx
 // Halo fill: the values boundary cells pull from outside the lattice (before the step).
 void launch_halo(int storage, int rep_s, const GridDesc& g, const FluidParams& fp, const FluidBuffers& b,
                  cudaStream_t s);
-// The fused kernel takes the lattice faces itself and the step has no halo
-// fill (k_bulk in FP32 / FP64).  Not with an outflow face, whose cells copy what
+// Faces that the fused FP32 / FP64 kernel takes itself (k_bulk): 0 none, 1 all
+// (the step has no halo fill), 2 far-field / velocity x faces (whose fill is one
+// scattered store per row and direction; the y and z faces' are contiguous
+// rows).  Not all with with an outflow face, whose cells copy what
 // their interior neighbours receive (slots the same launch overwrites), nor with
 // a geometry and a periodic face, where a cut link may cross the seam.  And only
 // on lattices of up to kInlineFaceCells cells, where the fill's launch counts:
 // measured per step, fill -> inline: periodic 24^3 11.3 -> 5.3 us, 64^3 16.5 ->
 // 11.6 (FP64 21.7 -> 17.0), 96^3 29.8 -> 24.9, 128^3 71.5 -> 70.1 (RR3 75.5 ->
 // 79.6), 192^3 235.7 -> 235.3; on 512 x 256 x 256 with far-field faces the boundary
-// warps cost more than the fill (1.24 -> 1.26 ms).
+// warps cost more than the fill (1.24 -> 1.26 ms), and the x faces alone less
+// (1.22 -> 1.15 ms with the fill on the y and z faces).
 constexpr int64_t kInlineFaceCells = 1500000;
-bool bulk_inline_faces(int storage, const GridDesc& g, const FluidParams& fp, bool geometry);
+int bulk_inline_faces(int storage, const GridDesc& g, const FluidParams& fp, bool geometry);
 // Equilibrium initialisation into representation E.
 void launch_init(int storage, int init_kind, float amplitude, const GridDesc& g, const FluidParams& fp,
                  const FluidBuffers& b, cudaStream_t s);
