@@ -147,20 +147,27 @@ struct bfx_sim {
     uint64_t timing_launches = 0;
     std::vector<void*> allocations;
     cudaEvent_t region[2] = {nullptr, nullptr};
-    // CUDA graphs of two consecutive steps, keyed by the representation the
-    // pair starts from (the launch sequence repeats with period two).
-    cudaGraphExec_t pair_graph[2] = {nullptr, nullptr};
-    uint64_t pair_launches[2] = {0, 0};
-    // single steps (an odd step count, one-step calls), same keying
-    cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
-    uint64_t step_launches[2] = {0, 0};
-    // pipelined pairs: each step's geometry was built during the previous
-    // step's fluid kernel, and each step builds the next one's the same way
-    cudaGraphExec_t pipe_graph[2] = {nullptr, nullptr};
-    uint64_t pipe_launches[2] = {0, 0};
+    // CUDA graphs of consecutive plain steps, keyed by the representation they
+    // start from (the launch sequence repeats with period two): one step, a
+    // pair, kLongSteps steps, and a pipelined pair, which takes its first step's
+    // geometry as built (during the previous step's fluid kernel) and builds the
+    // one after its last the same way.  A graph launch leaves the GPU idle for
+    // about 2 us, which a long graph pays once (64^3 periodic wave 10.0 -> 9.2 us
+    // a step); it is captured when pairs have replayed kLongAfter times, so
+    // short runs do not pay for it.  Pipelined pairs stay pairs: sixteen steps
+    // in one graph ran slower (coupled bird on 64^3 54.8 -> 56.6 us a step).
+    enum { kStepGraph, kPairGraph, kPipePairGraph, kLongGraph, kGraphKinds };
+    static constexpr int kLongSteps = 16;
+    static constexpr uint64_t kLongAfter = 32;
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        uint64_t launches = 0;
+    } graphs[kGraphKinds][2];
+    uint64_t pair_replays = 0;
     // side stream of the next step's geometry build, with its fork / join events
     cudaStream_t side = nullptr;
     // the adjoint's wing-frame tangent (one thread, 50 us) beside that build
+    // (created by the first adjoint)
     cudaStream_t tangent = nullptr;
     cudaEvent_t tangent_ev = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr, lists_ev = nullptr;
@@ -379,9 +386,10 @@ void encode_halo(bfx_sim* s, const FluidBuffers& fb, bool staged, cudaStream_t s
 // The cut-link and topology-event lists of a step's geometry, on the
 // simulation's stream or (pipelined path) the side stream beside the previous
 // step's fluid kernel.
-void encode_link_build(bfx_sim* s, uint8_t* mprev, uint8_t* mnext, cudaStream_t st, cudaEvent_t lists_done = nullptr) {
+void encode_link_build(bfx_sim* s, uint8_t* mprev, uint8_t* mnext, cudaStream_t st, cudaEvent_t lists_done = nullptr,
+                       cudaStream_t search = nullptr) {
     launch_link_build(s->cfg.geometry, s->cfg.link_rule, s->g, s->fp, s->box, geom_buffers(s, mprev, mnext), st,
-                      lists_done);
+                      lists_done, search);
     s->launches += link_build_launches(s->cfg.geometry, s->cfg.link_rule, s->fp, s->scan_blocks);
 }
 // The topology impulses of the step's events: they read the pre-step
@@ -392,9 +400,14 @@ void encode_topology(bfx_sim* s, uint8_t* mprev, uint8_t* mnext) {
                     fluid_buffers(s, mnext), s->stream);
     s->launches += 1;
 }
+// Both, in a step that was not prefetched: the impulses need the event list
+// alone, so they run beside the search for the link fractions.
 void encode_links(bfx_sim* s, uint8_t* mprev, uint8_t* mnext) {
-    encode_link_build(s, mprev, mnext, s->stream);
+    const bool beside = s->moving() && s->side != nullptr && link_search(s->cfg.geometry, s->cfg.link_rule, s->fp);
+    encode_link_build(s, mprev, mnext, s->stream, beside ? s->lists_ev : nullptr, beside ? s->side : nullptr);
+    if (beside) cudaEventRecord(s->join_ev, s->side);
     if (s->moving()) encode_topology(s, mprev, mnext);
+    if (beside) cudaStreamWaitEvent(s->stream, s->join_ev, 0);
 }
 
 // What a taped step records beside the fluid kernel's moments: the wing-frame
@@ -592,7 +605,7 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     }
 }
 
-// Replays (capturing on first use) the graph of `nsteps` (1 or 2) plain steps
+// Replays (capturing on first use) the graph of `nsteps` (1, 2 or kLongSteps) plain steps
 // for the current parity.  Host-side state (representation, mask index)
 // alternates with period two, so a pair graph leaves it where it started and
 // the single-step graph of each parity hands over to the other's.  A pipelined
@@ -601,10 +614,11 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
 int run_steps_graph(bfx_sim* s, int nsteps, bool pipelined = false) {
     s->hstate_fresh = false;
     const int key = s->rep_s;
-    cudaGraphExec_t* slot = pipelined ? &s->pipe_graph[key] : nsteps == 2 ? &s->pair_graph[key] : &s->step_graph[key];
-    uint64_t* count =
-        pipelined ? &s->pipe_launches[key] : nsteps == 2 ? &s->pair_launches[key] : &s->step_launches[key];
-    if (!*slot) {
+    const int kind = nsteps == 1   ? bfx_sim::kStepGraph
+                     : nsteps == 2 ? (pipelined ? bfx_sim::kPipePairGraph : bfx_sim::kPairGraph)
+                                   : bfx_sim::kLongGraph;
+    bfx_sim::StepGraph& g = s->graphs[kind][key];
+    if (!g.exec) {
         const int rep0 = s->rep_s, cur0 = s->cur;
         cudaGraph_t graph = nullptr;
         uint64_t before = s->launches;
@@ -614,25 +628,38 @@ int run_steps_graph(bfx_sim* s, int nsteps, bool pipelined = false) {
         e = cudaStreamEndCapture(s->stream, &graph);
         if (e != cudaSuccess) return cuda_fail(s, e, "graph capture end");
         // kernel nodes keep the priority of the stream they were captured on
-        e = cudaGraphInstantiate(slot, graph, cudaGraphInstantiateFlagUseNodePriority);
+        e = cudaGraphInstantiate(&g.exec, graph, cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) return cuda_fail(s, e, "graph instantiate");
-        *count = s->launches - before;
+        g.launches = s->launches - before;
         s->launches = before;
         // capture only recorded the steps: the host state advances at launch
         s->rep_s = rep0;
         s->cur = cur0;
     }
-    cudaError_t e = cudaGraphLaunch(*slot, s->stream);
+    cudaError_t e = cudaGraphLaunch(g.exec, s->stream);
     if (e != cudaSuccess) return cuda_fail(s, e, "graph launch");
-    s->launches += *count;
+    s->launches += g.launches;
+    if (nsteps == 2) s->pair_replays += 1;
     for (int i = 0; i < nsteps; ++i) {
         s->rep_s ^= 1;
         if (s->moving()) s->cur ^= 1;
     }
     return BFX_OK;
 }
-int run_pair_graph(bfx_sim* s) { return run_steps_graph(s, 2); }
+// Replays graphs over k .. limit - 1 while whole ones fit: long ones (not
+// pipelined) once pairs have replayed often enough, then pairs.  Leaves the next
+// step in k.
+int run_graphs(bfx_sim* s, uint64_t& k, uint64_t limit, bool pipelined = false) {
+    while (k + 2 <= limit) {
+        const bool whole = !pipelined && s->pair_replays >= bfx_sim::kLongAfter && k + bfx_sim::kLongSteps <= limit;
+        const int n = whole ? bfx_sim::kLongSteps : 2;
+        const int rc = run_steps_graph(s, n, pipelined);
+        if (rc != BFX_OK) return rc;
+        k += n;
+    }
+    return BFX_OK;
+}
 
 // `count` steps without capture, samples or tape.  Pipelined where possible:
 // every step but the last builds the next step's geometry beside its own fluid
@@ -642,18 +669,16 @@ int run_plain_steps(bfx_sim* s, uint64_t count) {
     uint64_t k = 0;
     if (s->graphs_enabled && !s->timing && !s->topo_mode && can_pipeline(s) && count > 1) {
         encode_step(s, 0, nullptr, 0, nullptr, nullptr, false, true);
-        for (k = 1; k + 2 < count; k += 2) {
-            const int rc = run_steps_graph(s, 2, true);
-            if (rc != BFX_OK) return rc;
-        }
+        k = 1;
+        const int rc = run_graphs(s, k, count - 1, true);
+        if (rc != BFX_OK) return rc;
         for (; k < count; ++k) encode_step(s, 0, nullptr, 0, nullptr, nullptr, true, k + 1 < count);
         return BFX_OK;
     }
-    if (s->graphs_enabled && !s->timing)
-        for (; k + 1 < count; k += 2) {
-            const int rc = run_pair_graph(s);
-            if (rc != BFX_OK) return rc;
-        }
+    if (s->graphs_enabled && !s->timing) {
+        const int rc = run_graphs(s, k, count);
+        if (rc != BFX_OK) return rc;
+    }
     for (; k < count; ++k) encode_step(s, 0, nullptr, 0);
     return BFX_OK;
 }
@@ -876,12 +901,9 @@ void bfx_destroy(bfx_sim* s) {
     for (auto e : s->ev_stop) cudaEventDestroy(e);
     for (auto e : s->region)
         if (e) cudaEventDestroy(e);
-    for (auto g : s->pair_graph)
-        if (g) cudaGraphExecDestroy(g);
-    for (auto g : s->step_graph)
-        if (g) cudaGraphExecDestroy(g);
-    for (auto g : s->pipe_graph)
-        if (g) cudaGraphExecDestroy(g);
+    for (auto& kind : s->graphs)
+        for (auto& g : kind)
+            if (g.exec) cudaGraphExecDestroy(g.exec);
     if (s->fork_ev) cudaEventDestroy(s->fork_ev);
     if (s->join_ev) cudaEventDestroy(s->join_ev);
     if (s->lists_ev) cudaEventDestroy(s->lists_ev);
@@ -935,8 +957,6 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
     // side stream for the pipelined geometry build (optional: without it the
     // steps run in order on the main stream)
     if (cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, side_priority) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&s->tangent, cudaStreamNonBlocking, side_priority) != cudaSuccess ||
-        cudaEventCreateWithFlags(&s->tangent_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->join_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->lists_ev, cudaEventDisableTiming) != cudaSuccess ||
@@ -1326,10 +1346,8 @@ int bfx_advance(bfx_sim* s, uint64_t steps, uint32_t batch_size, uint32_t flags,
             // batch remains after them; the last one or two run directly.
             encode_step(s, 0, nullptr, 0, nullptr, nullptr, false, true);
             k = 1;
-            for (; k + 2 < count; k += 2) {
-                int rc = run_steps_graph(s, 2, true);
-                if (rc != BFX_OK) return rc;
-            }
+            const int rc = run_graphs(s, k, count - 1, true);
+            if (rc != BFX_OK) return rc;
             for (; k < count; ++k) {
                 const bool last = k + 1 == count;
                 if (capture && last && last_batch) s->capture_slot = slot;
@@ -1338,12 +1356,10 @@ int bfx_advance(bfx_sim* s, uint64_t steps, uint32_t batch_size, uint32_t flags,
             }
         } else if (s->graphs_enabled && !record && !s->timing && !s->topo_mode) {
             uint64_t plain = capture && done + count == steps ? count - 1 : count;
-            for (; k + 1 < plain; k += 2) {
-                int rc = run_pair_graph(s);
-                if (rc != BFX_OK) return rc;
-            }
+            int rc = run_graphs(s, k, plain);
+            if (rc != BFX_OK) return rc;
             if (k < plain) {
-                int rc = run_steps_graph(s, 1);
+                rc = run_steps_graph(s, 1);
                 if (rc != BFX_OK) return rc;
                 ++k;
             }
@@ -2053,6 +2069,16 @@ int bfx_adjoint(bfx_sim* s, uint64_t steps, const bfx_adjoint_objective* objecti
         cudaError_t ee = mem.get(&(ptr), (bytes));                                  \
         if (ee != cudaSuccess) return fail(s, BFX_ERR_ALLOCATION, "adjoint work memory allocation failed"); \
     } while (0)
+    if (can_pipeline(s) && !s->tangent) {
+        int least = 0, greatest = 0;
+        cudaDeviceGetStreamPriorityRange(&least, &greatest);
+        if (cudaStreamCreateWithPriority(&s->tangent, cudaStreamNonBlocking, greatest) != cudaSuccess ||
+            cudaEventCreateWithFlags(&s->tangent_ev, cudaEventDisableTiming) != cudaSuccess) {
+            (void)cudaGetLastError();  // the taped steps run in order instead
+            if (s->tangent) cudaStreamDestroy(s->tangent);
+            s->tangent = nullptr;
+        }
+    }
     // snapshots: nseg interval starts + the final state
     char* snap_pops = nullptr;
     uint8_t* snap_mask = nullptr;
@@ -2190,7 +2216,7 @@ int bfx_adjoint(bfx_sim* s, uint64_t steps, const bfx_adjoint_objective* objecti
         // the tape holds link_slots links per step: cap the link list there (the
         // recomputation reproduces the forward pass, whose largest count it is)
         s->link_capacity = (uint32_t)link_slots;
-        const bool pipelined = can_pipeline(s) && !s->timing;
+        const bool pipelined = can_pipeline(s) && !s->timing && s->tangent != nullptr;
         for (uint64_t j = 0; j < len; ++j) {
             reps[j] = s->rep_s;
             const TapeSlot t = slot(j), next = slot(j + 1 < len ? j + 1 : j);

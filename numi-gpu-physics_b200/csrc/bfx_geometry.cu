@@ -2033,13 +2033,16 @@ static bool ray_links(int geometry, int link_rule, const FluidParams& fp) {
 static bool bisected_links(int geometry, const FluidParams& fp) {
     return fp.interpolated && (geometry == BFX_GEOMETRY_ELLIPSOID || geometry == BFX_GEOMETRY_FLAPPING_WING);
 }
+bool link_search(int geometry, int link_rule, const FluidParams& fp) {
+    return ray_links(geometry, link_rule, fp) || bisected_links(geometry, fp);
+}
 int link_build_launches(int geometry, int link_rule, const FluidParams& fp, int scan_blocks) {
     const int nseg = (scan_blocks + kScanSegment - 1) / kScanSegment;
-    return 3 + (nseg > kScanDirect) + (ray_links(geometry, link_rule, fp) || bisected_links(geometry, fp));
+    return 3 + (nseg > kScanDirect) + link_search(geometry, link_rule, fp);
 }
 
 void launch_link_build(int geometry, int link_rule, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,
-                       const GeomBuffers& gb, cudaStream_t s, cudaEvent_t lists_done) {
+                       const GeomBuffers& gb, cudaStream_t s, cudaEvent_t lists_done, cudaStream_t search) {
     GeomArgs a = make_geom(g, fp, box, gb, nullptr);
     dim3 grid, block;
     box_shape(box, grid, block);
@@ -2058,6 +2061,10 @@ void launch_link_build(int geometry, int link_rule, const GridDesc& g, const Flu
     if (gb.live_list) k_links_emit_live<<<live_grid, block, 0, s>>>(a, (int)grid.x, (int)grid.y, fraction);
     else k_links_emit<<<grid, block, 0, s>>>(a, fraction);
     if (lists_done) cudaEventRecord(lists_done, s);
+    if (search) {
+        cudaStreamWaitEvent(search, lists_done, 0);
+        s = search;
+    }
     if (ray) {
         const unsigned rblocks =
             (unsigned)std::max<int64_t>(1, std::min<int64_t>(4096, ((int64_t)gb.link_capacity * 16 + 127) / 128));

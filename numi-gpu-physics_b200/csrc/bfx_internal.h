@@ -175,9 +175,12 @@ void launch_classify(int geometry, int has_prev, const GridDesc& g, const FluidP
 // scan, emission, link fractions).  Reads only geometry: masks, keys, wall
 // field and mesh.
 // lists_done (optional) is recorded once the lists are written, before the
-// link fractions.
+// link fractions; with `search`, these run on that stream, after the event.
 void launch_link_build(int geometry, int link_rule, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,
-                       const GeomBuffers& gb, cudaStream_t s, cudaEvent_t lists_done = nullptr);
+                       const GeomBuffers& gb, cudaStream_t s, cudaEvent_t lists_done = nullptr,
+                       cudaStream_t search = nullptr);
+// The link fractions of this geometry need a search kernel (ray roots, bisections).
+bool link_search(int geometry, int link_rule, const FluidParams& fp);
 // Kernel launches of one launch_link_build call.
 int link_build_launches(int geometry, int link_rule, const FluidParams& fp, int scan_blocks);
 // Topology impulses of the event list into topo_partials; reads the pre-step
