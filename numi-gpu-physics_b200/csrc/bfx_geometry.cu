@@ -1406,11 +1406,24 @@ __global__ void __maxnreg__(56) k_scan_apply(const GeomArgs a, int nseg) {
     const int first = blockIdx.x * kScanSegment + kScanPerThread * threadIdx.x;
     uint32_t c[kScanPerThread];
     uint32_t mine = 0;
+    // whole runs in 16-byte loads and stores: a thread's 32 counts are one
+    // 128-byte line
+    const bool whole = first + kScanPerThread <= nb;
+    if (whole) {
 #pragma unroll
-    for (int k = 0; k < kScanPerThread; ++k) {
-        c[k] = first + k < nb ? counts[first + k] : 0u;
-        mine += c[k];
+        for (int k = 0; k < kScanPerThread; k += 4) {
+            const uint4 v = *(const uint4*)(counts + first + k);
+            c[k] = v.x;
+            c[k + 1] = v.y;
+            c[k + 2] = v.z;
+            c[k + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanPerThread; ++k) c[k] = first + k < nb ? counts[first + k] : 0u;
     }
+#pragma unroll
+    for (int k = 0; k < kScanPerThread; ++k) mine += c[k];
     // block-exclusive prefix of the thread sums
     uint32_t incl = mine;
     for (int o = 1; o < 32; o <<= 1) {
@@ -1433,8 +1446,18 @@ __global__ void __maxnreg__(56) k_scan_apply(const GeomArgs a, int nseg) {
     }
 #pragma unroll
     for (int k = 0; k < kScanPerThread; ++k) {
-        if (first + k < nb) offsets[first + k] = base;
-        base += c[k];
+        const uint32_t n = c[k];
+        c[k] = base;
+        base += n;
+    }
+    if (whole) {
+#pragma unroll
+        for (int k = 0; k < kScanPerThread; k += 4)
+            *(uint4*)(offsets + first + k) = make_uint4(c[k], c[k + 1], c[k + 2], c[k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanPerThread; ++k)
+            if (first + k < nb) offsets[first + k] = c[k];
     }
 }
 

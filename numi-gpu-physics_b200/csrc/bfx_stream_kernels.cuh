@@ -490,11 +490,11 @@ __global__ void __maxnreg__(StreamShape<COLL>::max_regs)
                 if (!(l ? vb : va)) continue;
                 float r = __fmaf_rn(Lanes<P2>::get(cd, l), inv_dscale, 1.0f);
                 r = r > 1.0e-8f ? r : 1.0e-8f;
+                const float inv = inv_dscale / r;  // one division: the regularized step is bound by issue
                 const uint32_t gl = gida + 32 * l;
                 a.density[gl] = r;
-                a.velocity[gl] = make_float4(Lanes<P2>::get(cmx, l) * inv_dscale / r,
-                                             Lanes<P2>::get(cmy, l) * inv_dscale / r,
-                                             Lanes<P2>::get(cmz, l) * inv_dscale / r, 0.0f);
+                a.velocity[gl] = make_float4(Lanes<P2>::get(cmx, l) * inv, Lanes<P2>::get(cmy, l) * inv,
+                                             Lanes<P2>::get(cmz, l) * inv, 0.0f);
             }
         }
         if (COLL != BFX_COLLISION_TRT) {
