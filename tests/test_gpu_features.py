@@ -36,6 +36,48 @@ def small_mesh_case(**kw):
     return cases.flapping_plates(**args)
 
 
+def advance_case(name):
+    if name == "wave":
+        return lattice(cases.shear_wave(n=20, viscosity=0.02, axis="y")[0])
+    if name == "wing":
+        cfg, wing = cases.flapping_wing(chord=6, cycle_steps=240, viscosity=0.02)
+        return Lattice(cfg, wing=wing)
+    if name == "channel":  # static, clear of the faces: fill beside the links
+        return lattice(*cases.ellipsoid_channel(nx=64, ny=32, nz=32, radii=(9.0, 5.0, 4.5), viscosity=0.02,
+                                                storage=L.STORAGE_F16_DEVIATION)[:3])
+    if name == "compact bird":
+        from bfx.simulation import BirdFlowSimulation
+        return BirdFlowSimulation(*cases.compact_bird(free_flight=True, n=64)).lattice
+    storage, collision, link_rule, faces = {
+        "f32 ray": (L.STORAGE_F32, L.COLLISION_TRT, L.LINK_RAY_ROOT, L.BC_FARFIELD),
+        "f64 linear": (L.STORAGE_F64, L.COLLISION_RR3, L.LINK_LINEAR, L.BC_FARFIELD),
+        "f16 limiter": (L.STORAGE_F16_DEVIATION, L.COLLISION_TRT_LIMITER, L.LINK_RAY_ROOT, L.BC_FARFIELD),
+        "bf16 periodic": (L.STORAGE_BF16_DEVIATION, L.COLLISION_TRT, L.LINK_RAY_ROOT, L.BC_PERIODIC)}[name]
+    cfg, rows, body, mesh = small_mesh_case(storage=storage, collision=collision, link_rule=link_rule)
+    cfg.face_bc[2:6] = [faces] * 4
+    return lattice(cfg, rows, body, mesh)
+
+
+@pytest.mark.parametrize("name", ["wave", "wing", "channel", "compact bird", "f32 ray", "f64 linear", "f16 limiter",
+                                  "bf16 periodic"])
+def test_batched_steps_equal_single_steps(name):
+    """Batches (pipelined geometry in every storage, pair graphs, and sixteen-step graphs once pairs
+    have replayed 32 times) against one-step calls: populations, loads and body bit for bit."""
+    steps = 101
+    batched, single = advance_case(name), advance_case(name)
+    batched.advance(steps - 1, batch_size=40)
+    batched.advance(1)
+    for _ in range(steps):
+        single.advance(1, batch_size=1)
+    assert batched.step_index()[0] == single.step_index()[0] == steps
+    assert np.array_equal(batched.populations(), single.populations())
+    a, b = batched.loads(), single.loads()
+    assert list(a.force) == list(b.force) and list(a.torque) == list(b.torque) and a.link_count == b.link_count
+    assert list(batched.body().position) == list(single.body().position)
+    for x, y in zip(batched.links(), single.links()):
+        assert np.array_equal(x, y)
+
+
 @pytest.mark.parametrize("storage", [L.STORAGE_F32, L.STORAGE_F16_DEVIATION])
 def test_batch_partition_invariance_is_bit_exact(storage):
     """16 steps as 16x1, 4x4 and 1x16 give identical populations and loads.
