@@ -529,7 +529,8 @@ typedef struct bfx_adjoint_result {
     double reverse_ms;              /* device time of the recomputation and the reverse sweep, from its first
                                        launch (the allocation of its work memory is not included) */
     uint64_t max_links;             /* largest cut-link count of the run */
-    uint64_t work_bytes;            /* device memory of snapshots, tape and adjoint fields */
+    uint64_t work_bytes;            /* device memory of snapshots, tape and adjoint fields; the handle keeps
+                                       up to 8 GiB of it for its next adjoint call, until bfx_destroy */
 } bfx_adjoint_result;
 
 BFX_API int bfx_adjoint(bfx_sim* sim, uint64_t steps, const bfx_adjoint_objective* objective,

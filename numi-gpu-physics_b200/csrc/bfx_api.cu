@@ -50,11 +50,18 @@ namespace bfx {
 void set_global_error(const std::string& message) { g_create_error = message; }
 }  // namespace bfx
 
+// Device memory an adjoint call leaves with its handle for the next one.
+struct WorkBlock {
+    void* p;
+    size_t bytes;
+};
+
 struct bfx_sim {
     bfx_config cfg{};
     bfx_bird bird{};
     bool has_bird = false;
     int device = 0;
+    std::vector<WorkBlock> adjoint_work;  // kept between adjoint calls (AdjointAllocs)
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     GridDesc g{};
@@ -896,6 +903,7 @@ void bfx_destroy(bfx_sim* s) {
         cudaSetDevice(s->device);
         cudaStreamSynchronize(s->stream);
     }
+    for (const WorkBlock& b : s->adjoint_work) cudaFree(b.p);
     for (void* p : s->allocations) cudaFree(p);
     for (auto e : s->ev_start) cudaEventDestroy(e);
     for (auto e : s->ev_stop) cudaEventDestroy(e);
@@ -1893,6 +1901,7 @@ int bfx_launch_count(bfx_sim* s, uint64_t* launches) {
 int bfx_device_bytes(bfx_sim* s, uint64_t* bytes) {
     if (!s || !bytes) return BFX_ERR_INVALID_ARGUMENT;
     *bytes = s->device_bytes;
+    for (const WorkBlock& b : s->adjoint_work) *bytes += b.bytes;
     return BFX_OK;
 }
 
@@ -1998,18 +2007,64 @@ int bfx_advance_ledger(bfx_sim* s, uint64_t steps, bfx_ledger_sample* samples, s
 
 namespace {
 
+// Work memory of one adjoint call.  Allocating and freeing some GB takes 5-250
+// ms of host time, varying from call to call, against 55 ms for the gradient
+// over 64 steps of 256 x 128 x 128; so a call leaves its blocks with the handle,
+// up to kAdjointKeep in all, and the next call takes those that fit.  Blocks
+// that a call does not use are freed at its end, a failed allocation frees the
+// kept ones and tries again, and bfx_destroy frees the rest.  The contents are
+// written before they are read, and every use is on the handle's streams.
+constexpr size_t kAdjointKeep = (size_t)8 << 30;
 struct AdjointAllocs {
-    std::vector<void*> ptrs;
+    explicit AdjointAllocs(bfx_sim* sim) : s(sim), kept(std::move(sim->adjoint_work)) {
+        s->adjoint_work.clear();
+        s->adjoint_work.reserve(32);  // more than a call's blocks: the destructor allocates nothing
+    }
+    AdjointAllocs(const AdjointAllocs&) = delete;
+    AdjointAllocs& operator=(const AdjointAllocs&) = delete;
+    bfx_sim* s;
+    std::vector<WorkBlock> kept, used;
     uint64_t bytes = 0;
+    void drop_kept() {
+        for (const WorkBlock& b : kept) cudaFree(b.p);
+        kept.clear();
+    }
     ~AdjointAllocs() {
-        for (void* p : ptrs) cudaFree(p);
+        drop_kept();
+        size_t held = 0;
+        for (const WorkBlock& b : used) {
+            if (held + b.bytes <= kAdjointKeep) {
+                held += b.bytes;
+                s->adjoint_work.push_back(b);
+            } else {
+                cudaFree(b.p);
+            }
+        }
     }
     template <class T>
     cudaError_t get(T** p, size_t n) {
         if (n == 0) n = 16;
+        // the smallest kept block that holds n without wasting a quarter of it
+        size_t best = kept.size();
+        for (size_t i = 0; i < kept.size(); ++i)
+            if (kept[i].bytes >= n && kept[i].bytes <= n + n / 4 + 4096 &&
+                (best == kept.size() || kept[i].bytes < kept[best].bytes))
+                best = i;
+        if (best < kept.size()) {
+            *p = (T*)kept[best].p;
+            used.push_back(kept[best]);
+            kept.erase(kept.begin() + (std::ptrdiff_t)best);
+            bytes += n;
+            return cudaSuccess;
+        }
         cudaError_t e = cudaMalloc((void**)p, n);
+        if (e == cudaErrorMemoryAllocation && !kept.empty()) {
+            (void)cudaGetLastError();
+            drop_kept();
+            e = cudaMalloc((void**)p, n);
+        }
         if (e == cudaSuccess) {
-            ptrs.push_back((void*)*p);
+            used.push_back({(void*)*p, n});
             bytes += n;
         }
         return e;
@@ -2063,7 +2118,7 @@ int bfx_adjoint(bfx_sim* s, uint64_t steps, const bfx_adjoint_objective* objecti
 
     const size_t pop_bytes = (size_t)19 * (size_t)s->g.padded * s->elem;
     const size_t n = (size_t)s->g.n;
-    AdjointAllocs mem;
+    AdjointAllocs mem(s);
 #define BFX_ADJ_ALLOC(ptr, bytes)                                                   \
     do {                                                                            \
         cudaError_t ee = mem.get(&(ptr), (bytes));                                  \

@@ -126,6 +126,24 @@ def test_adjoint_leaves_the_forward_state_and_objective():
     assert np.array_equal(lat.populations(), ref.populations())
 
 
+def test_repeated_adjoints_on_one_handle():
+    """Work memory kept from a longer call and from an equal one does not change a gradient."""
+    kept, fresh = build(storage=L.STORAGE_F32), build(storage=L.STORAGE_F32)
+    before = kept.device_bytes()
+    first = kept.adjoint(13, (0.0, 0.0, 1.0), 0.5)
+    assert kept.device_bytes() == before + first.work_bytes
+    second = kept.adjoint(8, (0.0, 0.0, 1.0), 0.5)
+    third = kept.adjoint(8, (0.0, 0.0, 1.0), 0.5)
+    fresh.advance(13)
+    want_second = fresh.adjoint(8, (0.0, 0.0, 1.0), 0.5)
+    fresh.close()
+    again = build(storage=L.STORAGE_F32)
+    again.advance(21)
+    want_third = again.adjoint(8, (0.0, 0.0, 1.0), 0.5)
+    for got, want in ((second, want_second), (third, want_third)):
+        assert got.objective == want.objective and list(got.gradient) == list(want.gradient)
+
+
 def test_torch_autograd_bridge():
     torch = pytest.importorskip("torch")
     from bfx.autograd import kinematic_objective
