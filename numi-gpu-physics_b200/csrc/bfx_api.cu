@@ -224,10 +224,23 @@ int cuda_fail(bfx_sim* s, cudaError_t e, const char* what) {
     return e == cudaErrorMemoryAllocation ? BFX_ERR_ALLOCATION : BFX_ERR_KERNEL;
 }
 
+// Device memory for the handle.  What an adjoint call left with it
+// (AdjointAllocs) is freed before an allocation is given up.
+cudaError_t handle_malloc(bfx_sim* s, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && !s->adjoint_work.empty()) {
+        (void)cudaGetLastError();
+        for (const WorkBlock& b : s->adjoint_work) cudaFree(b.p);
+        s->adjoint_work.clear();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 template <class T>
 cudaError_t dalloc(bfx_sim* s, T** p, size_t bytes) {
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMalloc((void**)p, bytes);
+    cudaError_t e = handle_malloc(s, (void**)p, bytes);
     if (e == cudaSuccess) {
         s->allocations.push_back((void*)*p);
         s->device_bytes += bytes;
@@ -1330,7 +1343,7 @@ int bfx_advance(bfx_sim* s, uint64_t steps, uint32_t batch_size, uint32_t flags,
     } slot_guard{s->slots.get(), slot};
     if (record && steps > s->dsamples_cap) {
         void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, steps * sizeof(bfx_run_sample));
+        cudaError_t e = handle_malloc(s, &p, steps * sizeof(bfx_run_sample));
         if (e != cudaSuccess) return cuda_fail(s, e, "run-sample allocation");
         if (s->dsamples) {
             cudaFree(s->dsamples);
@@ -1563,7 +1576,7 @@ int bfx_runtime_safety(bfx_sim* s, bfx_safety_record* out) {
 
 static int ensure_scratch(bfx_sim* s) {
     if (s->scratch_f32) return BFX_OK;
-    cudaError_t e = cudaMalloc(&s->scratch_f32, (size_t)19 * s->g.n * sizeof(float));
+    cudaError_t e = handle_malloc(s, (void**)&s->scratch_f32, (size_t)19 * s->g.n * sizeof(float));
     if (e != cudaSuccess) return cuda_fail(s, e, "read-out staging allocation");
     s->allocations.push_back(s->scratch_f32);
     return BFX_OK;
@@ -2012,7 +2025,8 @@ namespace {
 // over 64 steps of 256 x 128 x 128; so a call leaves its blocks with the handle,
 // up to kAdjointKeep in all, and the next call takes those that fit.  Blocks
 // that a call does not use are freed at its end, a failed allocation frees the
-// kept ones and tries again, and bfx_destroy frees the rest.  The contents are
+// kept ones and tries again (any other allocation of the handle too:
+// handle_malloc), and bfx_destroy frees the rest.  The contents are
 // written before they are read, and every use is on the handle's streams.
 constexpr size_t kAdjointKeep = (size_t)8 << 30;
 struct AdjointAllocs {
