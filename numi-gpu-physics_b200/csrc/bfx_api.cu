@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "../../include/bfx.h"
+#include "bfx_clearance.h"
 #include "bfx_internal.h"
 #include "bfx_observation.h"
 
@@ -133,7 +134,7 @@ struct bfx_sim {
     float* scratch_f32 = nullptr;  // canonical read-out staging (lazily)
     FaceEquilibria faces{};        // far-field / velocity face values of the fused kernel,
     int inline_faces = 0;          // and which of them it takes itself (bulk_inline_faces)
-    bool solid_clear = false;      // static geometry that stays clear of every face
+    bool solid_clear = false;      // static geometry clear of every face (kFaceClearance); a restore finds it anew
     int face_ready = 0;            // faces the staged kernel takes from face_dev without their fill: 0, 2 (x) or 6
     float face_dev[6 * 19] = {};   // their values (stored deviations, host copy)
     bfx_run_sample* dsamples = nullptr;
@@ -625,6 +626,15 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     }
 }
 
+// Frees the captured graphs; the next steps capture their own.
+void drop_graphs(bfx_sim* s) {
+    for (auto& kind : s->graphs)
+        for (auto& g : kind) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = {};
+        }
+}
+
 // Replays (capturing on first use) the graph of `nsteps` (1, 2 or kLongSteps) plain steps
 // for the current parity.  Host-side state (representation, mask index)
 // alternates with period two, so a pair graph leaves it where it started and
@@ -922,9 +932,7 @@ void bfx_destroy(bfx_sim* s) {
     for (auto e : s->ev_stop) cudaEventDestroy(e);
     for (auto e : s->region)
         if (e) cudaEventDestroy(e);
-    for (auto& kind : s->graphs)
-        for (auto& g : kind)
-            if (g.exec) cudaGraphExecDestroy(g.exec);
+    drop_graphs(s);
     if (s->fork_ev) cudaEventDestroy(s->fork_ev);
     if (s->join_ev) cudaEventDestroy(s->join_ev);
     if (s->lists_ev) cudaEventDestroy(s->lists_ev);
@@ -1114,7 +1122,8 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
         // geometry box
         float r = geometry_radius(&c, &s->bird, mesh);
         int half = (int)std::ceil(r / c.cell_size) + 4;
-        // r already holds two cells beyond the geometry
+        // r already holds two cells beyond the geometry: no solid cell within
+        // kFaceClearance cells of a face
         s->solid_clear = c.static_geometry != 0;
         for (int k = 0; k < 3; ++k) {
             const double at = (hs.body[k] - c.origin[k]) / c.cell_size, reach = r / c.cell_size;
@@ -1755,6 +1764,15 @@ int bfx_restore_state(bfx_sim* s, const void* buf, size_t size) {
     p += sizeof(DeviceState);
     if (e == cudaSuccess) e = cudaMemcpy(s->pops, p, (size_t)19 * s->g.padded * s->elem, cudaMemcpyHostToDevice);
     p += (size_t)19 * s->g.padded * s->elem;
+    if (s->geometry() && !s->moving()) {
+        // The geometry of the saved state need not lie where this handle's was
+        // created: whether the halo fill may run beside the links follows from
+        // the restored mask, and the graphs captured for the other case go.
+        const bool clear = solid_clear_of_faces((const uint8_t*)p + (size_t)h.cur * (size_t)s->g.n, s->g.nx, s->g.ny,
+                                                s->g.nz, kPartMask);
+        if (clear != s->solid_clear) drop_graphs(s);
+        s->solid_clear = clear;
+    }
     if (s->geometry()) {
         if (e == cudaSuccess) e = cudaMemcpy(s->mask[0], p, (size_t)s->g.n, cudaMemcpyHostToDevice);
         p += s->g.n;

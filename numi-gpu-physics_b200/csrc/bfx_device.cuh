@@ -323,9 +323,4 @@ __device__ __forceinline__ bool padded_shell_cell(const Grid& g, int64_t t, int&
     return false;
 }
 
-// Mask byte: bits 0-5 part id (0 = fluid), bit 6 newly uncovered, bit 7 newly covered.
-constexpr uint8_t kPartMask = 0x3F;
-constexpr uint8_t kUncovered = 0x40;
-constexpr uint8_t kCovered = 0x80;
-
 }  // namespace bfx

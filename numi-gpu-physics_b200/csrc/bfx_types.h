@@ -7,6 +7,11 @@
 
 namespace bfx {
 
+// Mask byte: bits 0-5 part id (0 = fluid), bit 6 newly uncovered, bit 7 newly covered.
+constexpr uint8_t kPartMask = 0x3F;
+constexpr uint8_t kUncovered = 0x40;
+constexpr uint8_t kCovered = 0x80;
+
 struct Grid;
 struct Spill;
 

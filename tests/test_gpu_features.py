@@ -218,6 +218,41 @@ def test_checkpoint_archive_round_trip_and_continuation(tmp_path):
     fresh.advance(1)  # the handle stays usable
 
 
+@pytest.mark.parametrize("how", ["restore_state", "from_archive"])
+@pytest.mark.parametrize("center", [(14.2, 1.3, 16.1), (44.9, 16.2, 30.6)])  # across y; outflow face and across z
+@pytest.mark.parametrize("storage", [L.STORAGE_F32, L.STORAGE_F16_DEVIATION])
+def test_restored_static_body_on_a_face_continues_like_the_original(storage, center, how, tmp_path):
+    """A static body restored into a handle that was created with its body clear of the faces (and
+    whose steps, graphs included, fill the halo beside the links) steps bit for bit like the handle
+    created in its place: there the fill must come before the links."""
+    def build(at):
+        cfg, rows, body, _ = cases.ellipsoid_channel(nx=48, ny=32, nz=32, radii=(4.0, 3.6, 3.8), center=at,
+                                                     viscosity=0.02, storage=storage, collision=L.COLLISION_TRT)
+        return lattice(cfg, rows, body)
+    clear = (14.0, 16.0, 16.0)
+    there = build(center)
+    there.advance(7)
+    if how == "restore_state":
+        state = there.save_state()
+        moved = build(clear)
+        moved.advance(80, batch_size=80)
+        moved.restore_state(state)
+    else:
+        body = there.body()
+        body.position[:] = list(clear)
+        there.set_body(body)  # static geometry: the occupancy stays
+        path = str(tmp_path / "moved")
+        there.save_archive(path)
+        moved = Lattice.from_archive(path)
+    assert np.array_equal(moved.mask(), there.mask())
+    for _ in range(3):
+        moved.advance(33, batch_size=33)
+        there.advance(33, batch_size=33)
+        assert np.array_equal(moved.populations(), there.populations())
+        a, b = moved.loads(), there.loads()
+        assert list(a.force) == list(b.force) and a.link_count == b.link_count > 0
+
+
 def test_corrupted_checkpoint_fails_cleanly():
     cfg, _, _, _ = cases.shear_wave(n=16, viscosity=0.03, magic=3.0 / 16.0, axis="y")
     lat = lattice(cfg)
