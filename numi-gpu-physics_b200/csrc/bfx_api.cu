@@ -387,18 +387,24 @@ bool halo_beside_links(const bfx_sim* s) {
     return s->moving() ? faces_constant(s->cfg) : s->solid_clear;
 }
 // Without geometry and without a body update the end of a step is its counter
-// alone: the fused kernel counts it (not BF16, whose stochastic stores read
-// the counter).
-bool step_counted_by_bulk(const bfx_sim* s) {
+// alone: the halo fill counts it, or the fused kernel where there is no fill
+// (not BF16, whose stochastic stores read the counter).  Counting in the fused
+// kernel beside a fill cost it more than the launch saved: the store before its
+// loads took 227 -> 236 us (TRT) and 428 -> 456 us (limiter) on a periodic 192^3
+// in FP32.
+bool step_counted(const bfx_sim* s) {
     return !s->geometry() && !(s->cfg.free_flight && s->has_bird) && s->cfg.storage != BFX_STORAGE_BF16_DEVIATION;
 }
 
-// The halo fill the step's fused kernel needs, on one stream: none where it
-// takes the faces itself, the y / z faces for the staged kernel with x-face
-// values or FP32 / FP64 with inline x faces, or every face.
+// The step has a halo fill: not where the fused kernel takes every face itself.
+bool halo_filled(const bfx_sim* s, bool staged) { return !(staged ? s->face_ready == 6 : s->inline_faces == 1); }
+
+// The halo fill the step's fused kernel needs, on one stream: the y / z faces
+// for the staged kernel with x-face values or FP32 / FP64 with inline x faces,
+// or every face.
 void encode_halo(bfx_sim* s, const FluidBuffers& fb, bool staged, cudaStream_t st) {
     const bool yz_only = staged ? s->face_ready != 0 : s->inline_faces == 2;
-    if (s->inline_faces == 1 || (staged && s->face_ready == 6)) return;
+    if (!halo_filled(s, staged)) return;
     if (yz_only) launch_halo_yz(s->cfg.storage, s->rep_s, s->g, s->fp, fb, st);
     else launch_halo(s->cfg.storage, s->rep_s, s->g, s->fp, fb, st);
     s->launches += 1;
@@ -496,6 +502,8 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     // The halo fill forks off here (after the previous step's fluid kernel)
     // and joins before this step's fluid kernel
     const bool staged = bulk_staged(s->cfg.storage, s->cfg.collision, tape ? 2 : capture, s->tma_ok);
+    const bool counted = step_counted(s), filled = halo_filled(s, staged);
+    fb.count_step = counted && filled ? 1 : 0;
     const bool halo_side = halo_beside_links(s) && !tape && !ledger_in;
     if (halo_side) {
         cudaEventRecord(s->halo_fork_ev, s->stream);
@@ -535,8 +543,7 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     const FinishParams fin = {{s->cfg.gravity[0], s->cfg.gravity[1], s->cfg.gravity[2]}, (int)s->cfg.body_substeps,
                               s->cfg.free_flight && s->has_bird ? 1 : 0};
     const bool finish_fused = s->geometry() && !tape;
-    const bool counted = step_counted_by_bulk(s);
-    fb.count_step = counted ? 1 : 0;
+    fb.count_step = counted && !filled ? 1 : 0;
     if (s->geometry()) {
         GeomBuffers gb = geom_buffers(s, mprev, mnext);
         if (tape) {

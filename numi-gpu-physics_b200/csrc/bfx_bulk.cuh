@@ -27,7 +27,7 @@ struct BulkArgs {
     float face_dev[6][19];
     int inline_faces;       // k_bulk takes faces itself: 0 none, 1 every face (load_cell_edge), 2 the x faces
     int skip_rare;          // k_bulk leaves solid / newly uncovered cells to k_rare (pipelined step)
-    int count_step;         // the fused kernel also counts the step (no end-of-step kernel)
+    int count_step;         // this launch (the halo fill, or the fused kernel without one) counts the step
     FaceEquilibria faces;
     int box[3];             // geometry box extent (origin in DeviceState); rare-cell launch
     void* pops;

@@ -480,8 +480,8 @@ __global__ void __launch_bounds__(256, sizeof(typename S::R) == 8 ? 1 : (COLL ==
     const uint32_t gid = (uint32_t)x + (uint32_t)a.g.nx * ((uint32_t)y + (uint32_t)a.g.ny * (uint32_t)z);
     const uint32_t pid =
         (uint32_t)(x + 1) + (uint32_t)a.g.px * ((uint32_t)(y + 1) + (uint32_t)a.g.py * (uint32_t)(z + 1));
-    // the step counter's only readers are the stochastic stores
-    if (!S::kStochastic && gid == 0 && a.count_step) a.state->step += 1;
+    // without a fill, which would count the step (no stochastic store reads the counter here)
+    if (FACES == 1 && gid == 0 && a.count_step) a.state->step += 1;
     if (a.mask) {
         const uint8_t m = a.mask[gid];
         if (m) {

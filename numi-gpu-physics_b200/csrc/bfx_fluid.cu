@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(128) k_halo(const BulkArgs a, int rep_s, int64
     using R = typename S::R;
     const Grid& g = a.g;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0 && a.count_step) a.state->step += 1;
     if (t >= halo_cells) return;
     int hx, hy, hz;
     if (!padded_shell_cell(g, t, hx, hy, hz)) return;

@@ -38,7 +38,7 @@ struct FluidBuffers {
     int sm_count;
     const FaceEquilibria* faces;  // host copy; null: the halo fill covers every face
     int inline_faces;       // faces k_bulk takes from them: 1 every face, 2 the x faces
-    int count_step;         // the fused kernel counts the step (no geometry, no body update)
+    int count_step;         // the launch counts the step (no geometry, no body update)
     const float* face_dev;  // host copy of the face values [6][19] for the staged kernel (null: the halo
                             // fill covers every face)
     int face_count;         // faces the staged kernel takes from face_dev: 2 (-x, +x) or 6

@@ -78,6 +78,25 @@ def test_batched_steps_equal_single_steps(name):
         assert np.array_equal(x, y)
 
 
+@pytest.mark.parametrize("storage", [L.STORAGE_F32, L.STORAGE_F64, L.STORAGE_F16_DEVIATION, L.STORAGE_BF16_DEVIATION])
+@pytest.mark.parametrize("collision", [L.COLLISION_TRT, L.COLLISION_TRT_LIMITER])
+@pytest.mark.parametrize("faces", ["pppppp", "ffffff", "ffpppp", "foffff"])
+@pytest.mark.parametrize("extent", [(20, 18, 17), (9, 200, 190)])
+def test_every_step_without_geometry_is_counted_once(storage, collision, faces, extent):
+    """The step counter without geometry, on each route: by the halo fill (all faces, or y and z), by
+    the fused kernels where they take every face, by the end-of-step kernel (BF16); in direct steps,
+    graphs and capturing steps."""
+    cfg, _, _, _ = cases.shear_wave(nx=extent[0], ny=extent[1], nz=extent[2], viscosity=0.03, storage=storage,
+                                    collision=collision)
+    cfg.face_bc[:] = [{"p": L.BC_PERIODIC, "f": L.BC_FARFIELD, "o": L.BC_OUTFLOW}[c] for c in faces]
+    lat = lattice(cfg)
+    for steps, done in ((1, 1), (6, 7), (75, 82)):
+        lat.advance(steps, batch_size=75)
+        assert lat.step_index()[0] == done
+    lat.advance(3, capture_fields=True)
+    assert lat.step_index()[0] == 85
+
+
 @pytest.mark.parametrize("storage", [L.STORAGE_F32, L.STORAGE_F16_DEVIATION])
 def test_batch_partition_invariance_is_bit_exact(storage):
     """16 steps as 16x1, 4x4 and 1x16 give identical populations and loads.
