@@ -1055,7 +1055,7 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
                         ? (int)std::ceil(c.mesh_half_thickness / c.cell_size) + 2 + 3
                         : (c.geometry == BFX_GEOMETRY_FLAPPING_WING ? 3 : 0);
 
-    s->inline_faces = bulk_inline_faces(c.storage, g, fp, c.geometry != BFX_GEOMETRY_NONE);
+    s->inline_faces = bulk_inline_faces(c.storage, c.collision, g, fp, c.geometry != BFX_GEOMETRY_NONE);
     if (s->inline_faces) s->faces = make_face_equilibria(fp);
 
     s->elem = storage_bytes(c.storage);

@@ -11,6 +11,8 @@
 // branch-free path: 19 loads, moments, collision, optional sponge, 19 stores
 // (152 B per cell in FP32, 76 B in the 16-bit formats).
 #define BFX_VARIANT exact
+#include <algorithm>
+
 #include "bfx_bulk_kernels.cuh"
 #include "bfx_stream.cuh"
 
@@ -318,9 +320,38 @@ FaceEquilibria make_face_equilibria(const FluidParams& fp) {
     return e;
 }
 
-int bulk_inline_faces(int storage, const GridDesc& g, const FluidParams& fp, bool geometry) {
+// What a step saves without its halo fill, in us.  Saved: the fill's launch, its
+// y / z part and, where the x faces are periodic, its scattered rows.  Spent: the
+// face arithmetic in every warp (32 cells of a row) that holds a cell on a face
+// -- all of them on a narrow lattice -- and in FP64 a slower kernel for every
+// cell.  The costs are least-squares fits to 33 lattices of 14 K to 1.5 M cells
+// (24^3 to 114^3, 5 x 500 x 500, 4096 x 16 x 16, ...) with periodic and far-field
+// faces, fill and inline measured in turn; the sign picks the faster one, or one
+// within 2 %, in 619 of 640 cases.  Per step, fill -> inline: FP32 TRT periodic 64^3
+// 12.9 -> 9.2, 112^3 46.8 -> 45.9, 33 x 150 x 150 35.3 -> 37.8, 5 x 500 x 500 171 -> 211;
+// FP64 RR3 64^3 21.7 -> 17.5, 112^3 102 -> 112; FP64 regularized 112^3 99.6 -> 91.2.
+double inline_face_gain(int storage, int collision, const GridDesc& g) {
+    struct Cost {
+        double row, edge, cell;  // per 1,000 x-periodic rows saved; per 1,000 edge warps and per million cells spent
+    };
+    // by collision: TRT, limiter, regularized, RR3
+    static const Cost f32[4] = {{0.10, 0.16, 0.0}, {0.10, 0.18, 0.0}, {0.04, 0.06, 0.0}, {0.06, 0.11, 0.0}};
+    static const Cost f64[4] = {{0.16, 0.17, 2.0}, {0.08, 0.12, 4.0}, {0.04, 0.04, 2.0}, {0.20, 0.22, 4.0}};
+    static_assert(BFX_COLLISION_TRT == 0 && BFX_COLLISION_TRT_LIMITER == 1 && BFX_COLLISION_REGULARIZED == 2 &&
+                      BFX_COLLISION_RR3 == 3,
+                  "the costs are listed in this order");
+    const Cost& c = (storage == BFX_STORAGE_F64 ? f64 : f32)[collision & 3];
+    const double per_row = (g.nx + 31) / 32, rows = (double)g.ny * g.nz;
+    const double inner = (double)std::max(g.ny - 2, 0) * std::max(g.nz - 2, 0);
+    const double edge_warps = inner * std::min(per_row, 2.0) + (rows - inner) * per_row;
+    return 4.7 + (g.per_x ? c.row * 1.0e-3 * rows : 0.0) + 0.036e-3 * g.nx * ((double)g.ny + g.nz) -
+           c.edge * 1.0e-3 * edge_warps - c.cell * 1.0e-6 * (double)g.n;
+}
+
+int bulk_inline_faces(int storage, int collision, const GridDesc& g, const FluidParams& fp, bool geometry) {
     if (storage != BFX_STORAGE_F32 && storage != BFX_STORAGE_F64) return 0;
-    bool every = g.n <= kInlineFaceCells, x_values = true;
+    bool every = g.n <= kInlineFaceCells && inline_face_gain(storage, collision, g) > 0.0;
+    bool x_values = true;
     for (int f = 0; f < 6; ++f) {
         const bool value = fp.face_bc[f] == BFX_BC_FARFIELD || fp.face_bc[f] == BFX_BC_VELOCITY;
         every = every && (value || (fp.face_bc[f] == BFX_BC_PERIODIC && !geometry));

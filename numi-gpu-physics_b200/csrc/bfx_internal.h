@@ -82,17 +82,15 @@ void launch_halo(int storage, int rep_s, const GridDesc& g, const FluidParams& f
 // Faces that the fused FP32 / FP64 kernel takes itself (k_bulk): 0 none, 1 all
 // (the step has no halo fill), 2 far-field / velocity x faces (whose fill is one
 // scattered store per row and direction; the y and z faces' are contiguous
-// rows).  Not all with with an outflow face, whose cells copy what
-// their interior neighbours receive (slots the same launch overwrites), nor with
-// a geometry and a periodic face, where a cut link may cross the seam.  And only
-// on lattices of up to kInlineFaceCells cells, where the fill's launch counts:
-// measured per step, fill -> inline: periodic 24^3 11.3 -> 5.3 us, 64^3 16.5 ->
-// 11.6 (FP64 21.7 -> 17.0), 96^3 29.8 -> 24.9, 128^3 71.5 -> 70.1 (RR3 75.5 ->
-// 79.6), 192^3 235.7 -> 235.3; on 512 x 256 x 256 with far-field faces the boundary
-// warps cost more than the fill (1.24 -> 1.26 ms), and the x faces alone less
-// (1.22 -> 1.15 ms with the fill on the y and z faces).
+// rows).  Never all with an outflow face, whose cells copy what their interior
+// neighbours receive (slots the same launch overwrites), nor with a geometry and
+// a periodic face, where a cut link may cross the seam.  All of them where
+// inline_face_gain (us a step) is positive, on up to kInlineFaceCells cells; above
+// nothing was measured to gain (512 x 256 x 256 with far-field faces 1.24 -> 1.26 ms,
+// the x faces alone 1.22 -> 1.15).
 constexpr int64_t kInlineFaceCells = 1500000;
-int bulk_inline_faces(int storage, const GridDesc& g, const FluidParams& fp, bool geometry);
+double inline_face_gain(int storage, int collision, const GridDesc& g);
+int bulk_inline_faces(int storage, int collision, const GridDesc& g, const FluidParams& fp, bool geometry);
 // Equilibrium initialisation into representation E.
 void launch_init(int storage, int init_kind, float amplitude, const GridDesc& g, const FluidParams& fp,
                  const FluidBuffers& b, cudaStream_t s);

@@ -97,6 +97,27 @@ def test_every_step_without_geometry_is_counted_once(storage, collision, faces, 
     assert lat.step_index()[0] == 85
 
 
+@pytest.mark.parametrize("extent,storage,collision,launches", [
+    ((64, 64, 64), L.STORAGE_F32, L.COLLISION_TRT, 1), ((4096, 16, 16), L.STORAGE_F32, L.COLLISION_RR3, 1),
+    ((8, 400, 400), L.STORAGE_F32, L.COLLISION_TRT, 2), ((33, 150, 150), L.STORAGE_F32, L.COLLISION_TRT_LIMITER, 2),
+    ((72, 72, 72), L.STORAGE_F64, L.COLLISION_RR3, 1), ((112, 112, 112), L.STORAGE_F64, L.COLLISION_RR3, 2),
+    ((96, 96, 96), L.STORAGE_F64, L.COLLISION_REGULARIZED, 1), ((128, 128, 128), L.STORAGE_F32, L.COLLISION_TRT, 2)])
+def test_faces_are_taken_by_the_kernel_where_few_warps_hold_one(extent, storage, collision, launches):
+    """One launch a step where the fused kernel takes the faces, two (with the fill) on lattices whose
+    warps mostly hold a face cell; a narrow and a wide cut of one shear wave agree either way."""
+    cfg, _, _, _ = cases.shear_wave(nx=extent[0], ny=extent[1], nz=extent[2], viscosity=0.03, storage=storage,
+                                    collision=collision, axis="z")
+    lat = lattice(cfg)
+    before = lat.launch_count()
+    lat.advance(6, batch_size=6)
+    assert lat.launch_count() - before == 6 * launches
+    small, _, _, _ = cases.shear_wave(nx=4, ny=4, nz=extent[2], viscosity=0.03, storage=storage,
+                                      collision=collision, axis="z")
+    ref = lattice(small)  # the wave depends on z alone
+    ref.advance(6, batch_size=6)
+    assert np.array_equal(lat.populations()[:, :, :4, :4], ref.populations())
+
+
 @pytest.mark.parametrize("storage", [L.STORAGE_F32, L.STORAGE_F16_DEVIATION])
 def test_batch_partition_invariance_is_bit_exact(storage):
     """16 steps as 16x1, 4x4 and 1x16 give identical populations and loads.
