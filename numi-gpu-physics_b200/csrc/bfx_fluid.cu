@@ -209,12 +209,17 @@ __global__ void k_macroscopic(const BulkArgs a, int rep_s) {
 }
 
 // FP64 mass and momentum of fluid cells in a fixed order (deterministic): a
-// warp takes whole lattice rows, and each thread keeps one FP64 sum per direction (19 additions a cell; mass and momentum are formed
-// from them once, with the products of the zero coefficients, so a non-finite
-// population shows in all four).  Then shuffles, and one single-block pass over
-// the block partials.  Bound by HBM; one cell a thread with integer divisions,
-// 133 FP64 operations and an FP64 shared-memory tree took 149 us for 319 MB
-// (256 x 128 x 128 FP32), this 70 us.
+// warp takes 64 consecutive cells at a time, and each thread keeps one FP64 sum
+// per direction (19 additions a cell; mass and momentum are formed from them
+// once, with the products of the zero coefficients, so a non-finite population
+// shows in all four).  Then shuffles, and one single-block pass over the block
+// partials.  Bound by HBM.  Consecutive cells rather than a warp per row: rows
+// need no division, but short ones leave lanes idle and few ones leave warps
+// idle.  The call, with its launch and read-back: 256 x 128 x 128 FP32 (319 MB)
+// 165 us with one cell a thread, 133 FP64 operations and a shared-memory tree, 81
+// by rows, 82 so (half storage 297, 74 and 77); 4 x 1024 x 1024 178, 514 and 126;
+// 512 x 11 x 11 30, 35 and 30.  Reciprocals with a fix-up in place of the two
+// divisions, or one pair of divisions per 64 cells, cost half storage 12 %.
 template <class S, int REP_S>
 __global__ void __launch_bounds__(256, 2) k_mass_momentum(const BulkArgs a, double* partials) {
     using T = typename S::T;
@@ -225,33 +230,32 @@ __global__ void __launch_bounds__(256, 2) k_mass_momentum(const BulkArgs a, doub
     double sum[19];
 #pragma unroll
     for (int q = 0; q < 19; ++q) sum[q] = 0.0;
-    const uint32_t rows = (uint32_t)g.ny * (uint32_t)g.nz;
-    for (uint32_t row = blockIdx.x * 8 + warp; row < rows; row += gridDim.x * 8) {
-        const int z = (int)(row / (uint32_t)g.ny), y = (int)(row - (uint32_t)z * (uint32_t)g.ny);
-        const uint32_t pid0 = (uint32_t)pflat(g, 0, y, z);
-        const uint8_t* mask = a.mask ? a.mask + (int64_t)row * g.nx : nullptr;
-        // two cells a lane at a time: 38 loads in flight
-        for (int x = lane; x < g.nx; x += 64) {
-            const int x2 = x + 32;
-            const bool in[2] = {!(mask && (mask[x] & kPartMask)), x2 < g.nx && !(mask && (mask[x2] & kPartMask))};
-            R v[2][19];
+    const uint32_t nx = (uint32_t)g.nx, ny = (uint32_t)g.ny;
+    const int64_t chunks = (g.n + 63) / 64;
+    for (int64_t chunk = (int64_t)blockIdx.x * 8 + warp; chunk < chunks; chunk += (int64_t)gridDim.x * 8) {
+        // two cells a lane: 38 loads in flight
+        R v[2][19];
+        bool in[2];
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const uint32_t pid = pid0 + (uint32_t)(c && x2 < g.nx ? x2 : x);
+        for (int c = 0; c < 2; ++c) {
+            const int64_t at = 64 * chunk + 32 * c + lane;
+            const uint32_t cell = (uint32_t)(at < g.n ? at : g.n - 1);
+            in[c] = at < g.n && !(a.mask && (a.mask[cell] & kPartMask));
+            const uint32_t row = cell / nx, z = row / ny;
+            const uint32_t pid = (uint32_t)pflat(g, (int)(cell - row * nx), (int)(row - z * ny), (int)z);
 #pragma unroll
-                for (int q = 0; q < 19; ++q) {
-                    // canon_load: A[opp q][x] (rep E) or A[q][x + c_q] (rep S)
-                    if (REP_S) v[c][q] = S::ld_rt((const T*)a.plane[q] + (uint32_t)(pid + (uint32_t)a.doff[q]), q);
-                    else v[c][q] = S::ld_rt((const T*)a.plane[opp(q)] + pid, opp(q));
-                }
+            for (int q = 0; q < 19; ++q) {
+                // canon_load: A[opp q][x] (rep E) or A[q][x + c_q] (rep S)
+                if (REP_S) v[c][q] = S::ld_rt((const T*)a.plane[q] + (uint32_t)(pid + (uint32_t)a.doff[q]), q);
+                else v[c][q] = S::ld_rt((const T*)a.plane[opp(q)] + pid, opp(q));
             }
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-                if (in[c]) {
-#pragma unroll
-                    for (int q = 0; q < 19; ++q) sum[q] += (double)v[c][q];
-                }
         }
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            if (in[c]) {
+#pragma unroll
+                for (int q = 0; q < 19; ++q) sum[q] += (double)v[c][q];
+            }
     }
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll

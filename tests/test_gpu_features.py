@@ -118,6 +118,36 @@ def test_faces_are_taken_by_the_kernel_where_few_warps_hold_one(extent, storage,
     assert np.array_equal(lat.populations()[:, :, :4, :4], ref.populations())
 
 
+@pytest.mark.parametrize("extent", [(4, 90, 101), (5, 4, 4), (31, 8, 9), (33, 7, 5), (63, 64, 3), (65, 9, 20), (256, 5, 4)])
+@pytest.mark.parametrize("storage", [L.STORAGE_F32, L.STORAGE_F64, L.STORAGE_F16_DEVIATION, L.STORAGE_BF16_DEVIATION])
+@pytest.mark.parametrize("steps", [2, 3])
+def test_mass_and_momentum_of_short_and_ragged_rows(extent, storage, steps):
+    """Both representations, rows around the 32 lanes and 64 cells of a warp's turn, few rows, solid
+    cells left out; and a non-finite population in all four sums."""
+    nx, ny, nz = (max(4, n) for n in extent)
+    cfg, rows, body, _ = cases.ellipsoid_channel(nx=nx, ny=ny, nz=nz, radii=(1.2, 1.1, 1.4), viscosity=0.03,
+                                                 center=(0.5 * nx, 0.5 * ny, 0.5 * nz), storage=storage,
+                                                 collision=L.COLLISION_TRT)
+    lat = lattice(cfg, rows, body)
+    lat.advance(steps)
+    pops = lat.populations().astype(np.float64)
+    fluid = (lat.mask().reshape(nz, ny, nx) & 0x3F) == 0
+    c = np.array([[0, 0, 0], [1, 0, 0], [-1, 0, 0], [0, 1, 0], [0, -1, 0], [0, 0, 1], [0, 0, -1], [1, 1, 0],
+                  [-1, -1, 0], [1, -1, 0], [-1, 1, 0], [1, 0, 1], [-1, 0, -1], [1, 0, -1], [-1, 0, 1], [0, 1, 1],
+                  [0, -1, -1], [0, 1, -1], [0, -1, 1]], dtype=np.float64)
+    sums = np.array([pops[q][fluid].sum() for q in range(19)])
+    want = np.concatenate([[sums.sum()], sums @ c])
+    # the read-out rounds FP64 populations to FP32
+    tolerance = 1e-12 if storage != L.STORAGE_F64 else 2.0 ** -24
+    assert np.max(np.abs(lat.mass_momentum() - want)) <= tolerance * want[0]
+    for value in (np.inf, np.nan):
+        bad = lat.populations()
+        bad[0][tuple(np.argwhere(fluid)[-1])] = value
+        lat.set_populations(bad)
+        got = lat.mass_momentum()
+        assert not np.isfinite(got).any(), got
+
+
 @pytest.mark.parametrize("storage", [L.STORAGE_F32, L.STORAGE_F16_DEVIATION])
 def test_batch_partition_invariance_is_bit_exact(storage):
     """16 steps as 16x1, 4x4 and 1x16 give identical populations and loads.
