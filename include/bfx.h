@@ -463,8 +463,15 @@ BFX_API int bfx_test_stall_staged_kernel(bfx_sim* sim, int32_t tile, uint32_t wa
 BFX_API int bfx_test_replay_topology(bfx_sim* sim, int mode, uint8_t* device_masks, uint64_t capacity_steps);
 /* Total kernel launches issued by the library on this handle. */
 BFX_API int bfx_launch_count(bfx_sim* sim, uint64_t* launches);
-/* Bytes of device memory held by the handle. */
+/* Bytes of device memory held by the handle, with the work memory its last
+ * gradient left for the next one (bfx_release_work_memory). */
 BFX_API int bfx_device_bytes(bfx_sim* sim, uint64_t* bytes);
+/* Frees the device memory that gradients (bfx_adjoint) on this handle's device
+ * left for the next ones: at most 8 GiB a device and a quarter of what was free
+ * when a gradient returned.  The library gives it back by itself before an
+ * allocation of any handle fails, and with the handle whose gradient left it;
+ * this call is for other allocators of the process. */
+BFX_API int bfx_release_work_memory(bfx_sim* sim);
 /* Allocation-free variant of bfx_fluid_mass_momentum.  It has no counterpart in
  * the reference.  It is for callers that cannot call cudaMalloc where they need
  * the sum: a host application whose device memory budget is already reserved
@@ -529,8 +536,8 @@ typedef struct bfx_adjoint_result {
     double reverse_ms;              /* device time of the recomputation and the reverse sweep, from its first
                                        launch (the allocation of its work memory is not included) */
     uint64_t max_links;             /* largest cut-link count of the run */
-    uint64_t work_bytes;            /* device memory of snapshots, tape and adjoint fields; the handle keeps
-                                       up to 8 GiB of it for its next adjoint call, until bfx_destroy */
+    uint64_t work_bytes;            /* device memory of snapshots, tape and adjoint fields; some of it is kept
+                                       for the next gradient (bfx_release_work_memory) */
 } bfx_adjoint_result;
 
 BFX_API int bfx_adjoint(bfx_sim* sim, uint64_t steps, const bfx_adjoint_objective* objective,

@@ -172,7 +172,7 @@ EXPORTED = (
     "bfx_last_error", "bfx_set_observation_buffers", "bfx_acquire_field_frame", "bfx_field_frame_copy",
     "bfx_release_field_frame", "bfx_release_field_frame_after", "bfx_capture_current_fields",
     "bfx_observation_counters", "bfx_flow_diagnostics", "bfx_create_flapping_wing", "bfx_test_stall_staged_kernel",
-    "bfx_test_replay_topology",
+    "bfx_test_replay_topology", "bfx_release_work_memory",
 )
 
 _lib = None
@@ -225,6 +225,7 @@ def load(path: str | None = None):
     L.bfx_timer_end.argtypes = [vp, P(ct.c_double)]
     L.bfx_launch_count.argtypes = [vp, P(ct.c_uint64)]
     L.bfx_device_bytes.argtypes = [vp, P(ct.c_uint64)]
+    L.bfx_release_work_memory.argtypes = [vp]
     L.bfx_fluid_mass_momentum_noalloc.argtypes = [vp, vp, ct.c_uint32, ct.c_uint32, ct.c_uint32, vp]
     L.bfx_adjoint.argtypes = [vp, ct.c_uint64, P(AdjointObjective), ct.c_uint32, P(AdjointResult)]
     L.bfx_advance_ledger.argtypes = [vp, ct.c_uint64, P(LedgerSample), ct.c_size_t, P(ct.c_uint64)]

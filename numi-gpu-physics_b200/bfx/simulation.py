@@ -509,6 +509,10 @@ class Lattice:
         _check(self.lib.bfx_device_bytes(self.handle, ct.byref(n)), self.handle)
         return n.value
 
+    def release_work_memory(self):
+        """Frees the device memory that gradients left for the next ones (for other allocators of the process)."""
+        _check(self.lib.bfx_release_work_memory(self.handle), self.handle)
+
 
 class BirdFlowSimulation:
     """BirdFlowSimulation (BirdFlowSimulation.swift:410-2096) on the CUDA backend.

@@ -19,6 +19,7 @@
 #include "bfx_clearance.h"
 #include "bfx_internal.h"
 #include "bfx_observation.h"
+#include "bfx_work_pool.h"
 
 using namespace bfx;
 
@@ -51,18 +52,11 @@ namespace bfx {
 void set_global_error(const std::string& message) { g_create_error = message; }
 }  // namespace bfx
 
-// Device memory an adjoint call leaves with its handle for the next one.
-struct WorkBlock {
-    void* p;
-    size_t bytes;
-};
-
 struct bfx_sim {
     bfx_config cfg{};
     bfx_bird bird{};
     bool has_bird = false;
     int device = 0;
-    std::vector<WorkBlock> adjoint_work;  // kept between adjoint calls (AdjointAllocs)
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     GridDesc g{};
@@ -225,18 +219,28 @@ int cuda_fail(bfx_sim* s, cudaError_t e, const char* what) {
     return e == cudaErrorMemoryAllocation ? BFX_ERR_ALLOCATION : BFX_ERR_KERNEL;
 }
 
-// Device memory for the handle.  What an adjoint call left with it
-// (AdjointAllocs) is freed before an allocation is given up.
-cudaError_t handle_malloc(bfx_sim* s, void** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && !s->adjoint_work.empty()) {
-        (void)cudaGetLastError();
-        for (const WorkBlock& b : s->adjoint_work) cudaFree(b.p);
-        s->adjoint_work.clear();
-        e = cudaMalloc(p, bytes);
-    }
-    return e;
+// The work memory that gradients leave for the next ones (bfx_work_pool.h): at
+// most kWorkKeep bytes a device, and at most a quarter of what the device has
+// free when a call ends.
+constexpr size_t kWorkKeep = (size_t)8 << 30;
+int device_allocate(void** p, size_t n) {
+    const cudaError_t e = cudaMalloc(p, n);
+    if (e != cudaSuccess) (void)cudaGetLastError();  // the caller reports it
+    return (int)e;
 }
+void device_release(void* p) { cudaFree(p); }
+WorkPool g_work({device_allocate, device_release, (int)cudaErrorMemoryAllocation});
+size_t work_limit() {
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return std::min(kWorkKeep, free_bytes / 4);
+}
+
+// Device memory for the handle.
+cudaError_t handle_malloc(bfx_sim* s, void** p, size_t bytes) { return (cudaError_t)g_work.allocate(s->device, p, bytes); }
 
 template <class T>
 cudaError_t dalloc(bfx_sim* s, T** p, size_t bytes) {
@@ -933,7 +937,7 @@ void bfx_destroy(bfx_sim* s) {
         cudaSetDevice(s->device);
         cudaStreamSynchronize(s->stream);
     }
-    for (const WorkBlock& b : s->adjoint_work) cudaFree(b.p);
+    g_work.drop(s);
     for (void* p : s->allocations) cudaFree(p);
     for (auto e : s->ev_start) cudaEventDestroy(e);
     for (auto e : s->ev_stop) cudaEventDestroy(e);
@@ -1938,8 +1942,14 @@ int bfx_launch_count(bfx_sim* s, uint64_t* launches) {
 
 int bfx_device_bytes(bfx_sim* s, uint64_t* bytes) {
     if (!s || !bytes) return BFX_ERR_INVALID_ARGUMENT;
-    *bytes = s->device_bytes;
-    for (const WorkBlock& b : s->adjoint_work) *bytes += b.bytes;
+    *bytes = s->device_bytes + g_work.held(s);
+    return BFX_OK;
+}
+
+int bfx_release_work_memory(bfx_sim* s) {
+    if (!s) return BFX_ERR_INVALID_ARGUMENT;
+    cudaSetDevice(s->device);
+    g_work.drain(s->device);
     return BFX_OK;
 }
 
@@ -2045,71 +2055,6 @@ int bfx_advance_ledger(bfx_sim* s, uint64_t steps, bfx_ledger_sample* samples, s
 
 namespace {
 
-// Work memory of one adjoint call.  Allocating and freeing some GB takes 5-250
-// ms of host time, varying from call to call, against 55 ms for the gradient
-// over 64 steps of 256 x 128 x 128; so a call leaves its blocks with the handle,
-// up to kAdjointKeep in all, and the next call takes those that fit.  Blocks
-// that a call does not use are freed at its end, a failed allocation frees the
-// kept ones and tries again (any other allocation of the handle too:
-// handle_malloc), and bfx_destroy frees the rest.  The contents are
-// written before they are read, and every use is on the handle's streams.
-constexpr size_t kAdjointKeep = (size_t)8 << 30;
-struct AdjointAllocs {
-    explicit AdjointAllocs(bfx_sim* sim) : s(sim), kept(std::move(sim->adjoint_work)) {
-        s->adjoint_work.clear();
-        s->adjoint_work.reserve(32);  // more than a call's blocks: the destructor allocates nothing
-    }
-    AdjointAllocs(const AdjointAllocs&) = delete;
-    AdjointAllocs& operator=(const AdjointAllocs&) = delete;
-    bfx_sim* s;
-    std::vector<WorkBlock> kept, used;
-    uint64_t bytes = 0;
-    void drop_kept() {
-        for (const WorkBlock& b : kept) cudaFree(b.p);
-        kept.clear();
-    }
-    ~AdjointAllocs() {
-        drop_kept();
-        size_t held = 0;
-        for (const WorkBlock& b : used) {
-            if (held + b.bytes <= kAdjointKeep) {
-                held += b.bytes;
-                s->adjoint_work.push_back(b);
-            } else {
-                cudaFree(b.p);
-            }
-        }
-    }
-    template <class T>
-    cudaError_t get(T** p, size_t n) {
-        if (n == 0) n = 16;
-        // the smallest kept block that holds n without wasting a quarter of it
-        size_t best = kept.size();
-        for (size_t i = 0; i < kept.size(); ++i)
-            if (kept[i].bytes >= n && kept[i].bytes <= n + n / 4 + 4096 &&
-                (best == kept.size() || kept[i].bytes < kept[best].bytes))
-                best = i;
-        if (best < kept.size()) {
-            *p = (T*)kept[best].p;
-            used.push_back(kept[best]);
-            kept.erase(kept.begin() + (std::ptrdiff_t)best);
-            bytes += n;
-            return cudaSuccess;
-        }
-        cudaError_t e = cudaMalloc((void**)p, n);
-        if (e == cudaErrorMemoryAllocation && !kept.empty()) {
-            (void)cudaGetLastError();
-            drop_kept();
-            e = cudaMalloc((void**)p, n);
-        }
-        if (e == cudaSuccess) {
-            used.push_back({(void*)*p, n});
-            bytes += n;
-        }
-        return e;
-    }
-};
-
 int adjoint_scope(bfx_sim* s) {
     const bfx_config& c = s->cfg;
     if (c.geometry != BFX_GEOMETRY_MESH || c.static_geometry)
@@ -2157,11 +2102,10 @@ int bfx_adjoint(bfx_sim* s, uint64_t steps, const bfx_adjoint_objective* objecti
 
     const size_t pop_bytes = (size_t)19 * (size_t)s->g.padded * s->elem;
     const size_t n = (size_t)s->g.n;
-    AdjointAllocs mem(s);
+    WorkCall mem(g_work, s->device, s);  // the contents are written before they are read
 #define BFX_ADJ_ALLOC(ptr, bytes)                                                   \
     do {                                                                            \
-        cudaError_t ee = mem.get(&(ptr), (bytes));                                  \
-        if (ee != cudaSuccess) return fail(s, BFX_ERR_ALLOCATION, "adjoint work memory allocation failed"); \
+        if (mem.get(&(ptr), (bytes)) != 0) return fail(s, BFX_ERR_ALLOCATION, "adjoint work memory allocation failed"); \
     } while (0)
     if (can_pipeline(s) && !s->tangent) {
         int least = 0, greatest = 0;
@@ -2371,8 +2315,9 @@ int bfx_adjoint(bfx_sim* s, uint64_t steps, const bfx_adjoint_objective* objecti
         result->forward_ms = f_ms;
         result->reverse_ms = r_ms;
         result->max_links = (uint64_t)ob.max_links;
-        result->work_bytes = mem.bytes;
+        result->work_bytes = mem.bytes();
     }
+    mem.keep(work_limit());  // idle: the streams were joined and synchronised above
     return BFX_OK;
 }
 

@@ -144,6 +144,26 @@ def test_repeated_adjoints_on_one_handle():
         assert got.objective == want.objective and list(got.gradient) == list(want.gradient)
 
 
+def test_work_memory_is_shared_and_given_back():
+    """A gradient leaves its work memory to the next one of any handle; a gradient that does not fit
+    frees it all and leaves the handle usable; a call gives it back."""
+    a, b = build(storage=L.STORAGE_F32), build(storage=L.STORAGE_F32)
+    a.release_work_memory()
+    held_a, held_b = a.device_bytes(), b.device_bytes()
+    first = a.adjoint(8, (0.0, 0.0, 1.0), 0.5)
+    assert a.device_bytes() == held_a + first.work_bytes
+    second = b.adjoint(8, (0.0, 0.0, 1.0), 0.5)
+    assert a.device_bytes() == held_a and b.device_bytes() == held_b + first.work_bytes
+    assert second.objective == first.objective and list(second.gradient) == list(first.gradient)
+    with pytest.raises(BirdFlowError, match="work memory"):
+        b.adjoint(10 ** 6, (0.0, 0.0, 1.0), 0.5, checkpoint_interval=1)  # a million snapshots
+    assert b.device_bytes() == held_b
+    third, fourth = b.adjoint(8, (0.0, 0.0, 1.0), 0.5), a.adjoint(8, (0.0, 0.0, 1.0), 0.5)
+    assert third.objective == fourth.objective and list(third.gradient) == list(fourth.gradient)
+    b.release_work_memory()
+    assert a.device_bytes() == held_a and b.device_bytes() == held_b
+
+
 def test_torch_autograd_bridge():
     torch = pytest.importorskip("torch")
     from bfx.autograd import kinematic_objective
