@@ -269,7 +269,7 @@ __device__ DV closest_point_dual(V3 p, const DV& a, const DV& b, const DV& c, Du
         return b;
     }
     const Du vc = d1 * d4 - d3 * d2;
-    if (vc.v <= 0.0f && d1.v >= 0.0f && d3.v <= 0.0f) {
+    if (vc.v <= 0.0f && d1.v >= 0.0f && d3.v <= 0.0f && d1.v > d3.v) {
         const Du v = d1 / (d1 - d3);
         bary[0] = dc(1.0f) - v;
         bary[1] = v;
@@ -285,7 +285,7 @@ __device__ DV closest_point_dual(V3 p, const DV& a, const DV& b, const DV& c, Du
         return c;
     }
     const Du vb = d5 * d2 - d1 * d6;
-    if (vb.v <= 0.0f && d2.v >= 0.0f && d6.v <= 0.0f) {
+    if (vb.v <= 0.0f && d2.v >= 0.0f && d6.v <= 0.0f && d2.v > d6.v) {
         const Du w = d2 / (d2 - d6);
         bary[0] = dc(1.0f) - w;
         bary[1] = dc(0.0f);
@@ -294,7 +294,7 @@ __device__ DV closest_point_dual(V3 p, const DV& a, const DV& b, const DV& c, Du
     }
     const Du va = d3 * d6 - d5 * d4;
     const Du e1 = d4 - d3, e2 = d5 - d6;
-    if (va.v <= 0.0f && e1.v >= 0.0f && e2.v >= 0.0f) {
+    if (va.v <= 0.0f && e1.v >= 0.0f && e2.v >= 0.0f && e1.v + e2.v > 0.0f) {
         const Du w = e1 / (e1 + e2);
         bary[0] = dc(0.0f);
         bary[1] = dc(1.0f) - w;

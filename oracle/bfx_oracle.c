@@ -1471,6 +1471,8 @@ float or_powf(float b, float e) { return bfx_powf(b, e); }
 /* Triangle mesh: closest point BF.metal:1529-1583; raster 1638-1686;  */
 /* resolve 1697-1738/1978-2039; links 2044-2076.                        */
 /* ------------------------------------------------------------------ */
+/* An edge region needs an edge of nonzero length: the reference divides 0 by 0
+ * there (two coincident vertices); here the following regions hold the point. */
 static void closest_point(const float p[3], const float a[3], const float b[3], const float c[3], float out[3],
                           float bary[3]) {
     float ab[3] = {b[0] - a[0], b[1] - a[1], b[2] - a[2]};
@@ -1490,7 +1492,7 @@ static void closest_point(const float p[3], const float a[3], const float b[3], 
         return;
     }
     float vc = d1 * d4 - d3 * d2;
-    if (vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f) {
+    if (vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f && d1 > d3) {
         float v = d1 / (d1 - d3);
         for (int k = 0; k < 3; ++k) out[k] = a[k] + v * ab[k];
         bary[0] = 1.0f - v; bary[1] = v; bary[2] = 0;
@@ -1504,14 +1506,14 @@ static void closest_point(const float p[3], const float a[3], const float b[3], 
         return;
     }
     float vb = d5 * d2 - d1 * d6;
-    if (vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f) {
+    if (vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f && d2 > d6) {
         float w = d2 / (d2 - d6);
         for (int k = 0; k < 3; ++k) out[k] = a[k] + w * ac[k];
         bary[0] = 1.0f - w; bary[1] = 0; bary[2] = w;
         return;
     }
     float va = d3 * d6 - d5 * d4;
-    if (va <= 0.0f && (d4 - d3) >= 0.0f && (d5 - d6) >= 0.0f) {
+    if (va <= 0.0f && (d4 - d3) >= 0.0f && (d5 - d6) >= 0.0f && (d4 - d3) + (d5 - d6) > 0.0f) {
         float w = (d4 - d3) / ((d4 - d3) + (d5 - d6));
         for (int k = 0; k < 3; ++k) out[k] = b[k] + w * (c[k] - b[k]);
         bary[0] = 0; bary[1] = 1.0f - w; bary[2] = w;

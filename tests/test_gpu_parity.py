@@ -490,3 +490,40 @@ def test_raster_matches_oracle(n_chord, n_span, shuffled):
         assert near.sum() > 500
         assert np.array_equal(wall[near], owall[near])
     assert compare_pops(lat, osim, "populations")[1]
+
+
+@pytest.mark.parametrize("link_rule", [L.LINK_LINEAR, L.LINK_RAY_ROOT])
+def test_triangles_without_area_match_oracle(link_rule):
+    """Triangles with two or three coincident vertices (by index and by position, in every order,
+    before and after the proper ones) own cells by their edge's distance: masks, walls, links and
+    populations equal the oracle's, hold no NaN, and repeat."""
+    cfg, rows, body, mesh = cases.flapping_plates(nx=72, ny=64, nz=56, span=17.3, chord=6.1, thickness=2.0,
+                                                  n_chord=8, n_span=24, period=300.0, viscosity=0.02,
+                                                  sponge_width=6.0, link_rule=link_rule)
+    tris, parts = np.asarray(mesh["tris"]), np.asarray(mesh["tri_part"])
+    nv = len(mesh["local"])
+    twin = tris[:, 1] + nv  # a copy of the second vertex
+    flat = np.concatenate([np.stack([tris[:, p[0]], tris[:, p[1]], tris[:, p[2]]], 1)[k::7]
+                           for k, p in enumerate([(0, 0, 1), (0, 1, 0), (1, 0, 0), (2, 2, 2)])] +
+                          [np.stack([tris[:, 1], twin, tris[:, 0]], 1)[4::7],
+                           np.stack([tris[:, 0], tris[:, 1], twin], 1)[5::7],
+                           np.stack([twin, tris[:, 2], tris[:, 1]], 1)[6::7]])
+    flat_part = np.concatenate([parts[k::7] for k in range(7)])
+    half = len(flat) // 2
+    mesh = dict(mesh, local=np.concatenate([mesh["local"]] * 2), segment=np.concatenate([mesh["segment"]] * 2),
+                tris=np.concatenate([flat[:half], tris, flat[half:]]).astype(np.uint32),
+                tri_part=np.concatenate([flat_part[:half], parts, flat_part[half:]]).astype(np.uint8))
+    lat, osim = make_pair(cfg, rows, body, mesh)
+    again = Lattice(cfg, bird_struct(rows), body_struct_from_tuple(body), mesh)
+    for step in range(3):
+        lat.advance(1)
+        again.advance(1)
+        osim.step()
+        assert np.array_equal(lat.mask(), osim.mcur)
+        wall, owall = lat.wall(), osim.wall.reshape(-1, 4)
+        near = np.abs(owall[:, 3]) < 1.9
+        assert near.sum() > 500 and np.isfinite(wall).all()
+        assert np.array_equal(wall[near], owall[near])
+        assert np.array_equal(again.wall(), wall) and np.array_equal(again.mask(), lat.mask())
+    assert compare_pops(lat, osim, "populations")[1]
+    assert np.isfinite(lat.populations()).all()
