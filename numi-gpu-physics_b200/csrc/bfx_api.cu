@@ -637,6 +637,14 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
     }
 }
 
+// The device state's occupancy need not be that of the handle's own last pose:
+// the next step's active bounds of a prescribed wing are open (k_prepare_wing).
+cudaError_t open_bounds_once(bfx_sim* s) {
+    if (s->cfg.geometry != BFX_GEOMETRY_FLAPPING_WING || !s->moving()) return cudaSuccess;
+    const int32_t mark = kOpenOnce;
+    return cudaMemcpy((char*)s->dstate + offsetof(DeviceState, act_lo), &mark, sizeof(mark), cudaMemcpyHostToDevice);
+}
+
 // Frees the captured graphs; the next steps capture their own.
 void drop_graphs(bfx_sim* s) {
     for (auto& kind : s->graphs)
@@ -1772,6 +1780,7 @@ int bfx_restore_state(bfx_sim* s, const void* buf, size_t size) {
     // a restored state never carries the staged kernel's test hook
     if (e == cudaSuccess)
         e = cudaMemset((char*)s->dstate + offsetof(DeviceState, test_stall_tile1), 0, 2 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = open_bounds_once(s);
     p += sizeof(DeviceState);
     if (e == cudaSuccess) e = cudaMemcpy(s->pops, p, (size_t)19 * s->g.padded * s->elem, cudaMemcpyHostToDevice);
     p += (size_t)19 * s->g.padded * s->elem;
@@ -1884,6 +1893,8 @@ int bfx_test_replay_topology(bfx_sim* s, int mode, uint8_t* device_masks, uint64
         return fail(s, BFX_ERR_INVALID_ARGUMENT, "record and replay need a device buffer of capacity_steps masks");
     const int rc = sync_check(s, "topology replay");
     if (rc != BFX_OK) return rc;
+    const cudaError_t e = open_bounds_once(s);  // replayed masks may be another wing's
+    if (e != cudaSuccess) return cuda_fail(s, e, "topology replay");
     s->topo_mode = mode;
     s->topo_buf = mode ? device_masks : nullptr;
     s->topo_cap = mode ? capacity_steps : 0;

@@ -478,7 +478,8 @@ __device__ void wing_pitch(float phase, const WingRec& w, float& angle, float& r
 // bounds: cells solid now or at the step before lie inside, and the link count,
 // the emission and the solid cells' kernel skip the rest (the count alone took
 // 96 of 305 us a step on a 16-cell chord).  Not with a planform whose chord has
-// no bound (negative beta exponent), nor with the occupancy test hook.
+// no bound (negative beta exponent), nor with the occupancy test hook, nor in the
+// first step after a restore, whose occupancy may be another wing's (kOpenOnce).
 __global__ void k_prepare_wing(const GeomArgs a, int init, float dt) {
     if (threadIdx.x > 1) return;
     DeviceState* st = a.b.state;
@@ -509,7 +510,7 @@ __global__ void k_prepare_wing(const GeomArgs a, int init, float dt) {
         const float lead = -0.25f * w.root_and_chord[3];
         const float trail = lead + w.root_and_chord[3] * w.geometry[3] * bfx_powf(0.25f, w.geometry[2]);
         const float half = 0.5f * fmaxf(w.geometry[1], a.fp.dx);
-        const bool open = !(w.geometry[2] >= 0.0f) || a.b.open_bounds;
+        const bool open = !(w.geometry[2] >= 0.0f) || a.b.open_bounds || st->act_lo[0] == kOpenOnce;
         for (int k = 0; k < 3; ++k) {
             const float root = w.root_and_chord[k], s = k == 0 ? sp.x : (k == 1 ? sp.y : sp.z),
                         c = k == 0 ? ch.x : (k == 1 ? ch.y : ch.z), n = k == 0 ? normal.x : (k == 1 ? normal.y : normal.z);

@@ -52,6 +52,10 @@ struct SegmentFrame {
     float4 origin, chord, span, normal, omega, uvel;
 };
 
+// act_lo[0] of a state whose occupancy need not be that of the handle's own last
+// pose (a restored one): the next step's bounds are open.
+constexpr int32_t kOpenOnce = -(1 << 30) - 1;
+
 // Device-resident per-simulation state updated by the single-thread kernels.
 struct DeviceState {
     uint64_t step;                 // completed steps
@@ -59,8 +63,9 @@ struct DeviceState {
     Prepared prep;
     int32_t box_origin[3];         // geometry region origin (cells)
     float geom_time;               // time (s) of the step the geometry was built for
-    // bounding box (cells, inclusive) of this step's mesh vertices; open
-    // (+-2^30) for the analytic shapes, empty before the vertices are placed
+    // bounding box (cells, inclusive) of this step's mesh vertices, or of the
+    // prescribed wing at this step and the last; open (+-2^30) for the other
+    // shapes, empty before the vertices are placed
     int32_t act_lo[3], act_hi[3];
     float wing_prev[16];           // GPUWingMomentumState
     float wing_reaction[16];       // GPUWingInertialReaction

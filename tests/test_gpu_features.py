@@ -323,6 +323,48 @@ def test_restored_static_body_on_a_face_continues_like_the_original(storage, cen
         assert list(a.force) == list(b.force) and a.link_count == b.link_count > 0
 
 
+@pytest.mark.parametrize("storage", [L.STORAGE_F32, L.STORAGE_F16_DEVIATION])
+@pytest.mark.parametrize("batch", [1, 4])
+def test_restored_wing_of_another_stroke_uncovers_the_old_cells(storage, batch):
+    """A state restored into a handle whose wing moves otherwise: the cells solid in the state lie
+    outside both poses the handle knows, and its next step must still uncover them.  Against the same
+    steps with the whole box active (the occupancy recorder keeps it so)."""
+    torch = pytest.importorskip("torch")
+
+    def build(amplitude_factor):
+        cfg, wing = cases.flapping_wing(chord=6, cycle_steps=240, viscosity=0.02, storage=storage)
+        wing.kinematics0.v[1] *= amplitude_factor
+        return Lattice(cfg, wing=wing)
+    first = build(1.0)
+    first.advance(20)
+    state = first.save_state()
+    got, want = build(0.4), build(0.4)
+    buf = torch.zeros(8 * got.n, dtype=torch.uint8, device="cuda")
+    want.replay_topology(1, buf.data_ptr(), 8)
+    for lat in (got, want):
+        lat.restore_state(state)
+    solid = first.mask() & 0x3F
+    for k in range(2):
+        got.advance(batch, batch_size=batch)
+        for _ in range(batch):
+            want.advance(1, batch_size=1)
+            if k == 0 and want.step_index()[0] == 21:
+                uncovered = want.loads().uncovered_count
+                assert uncovered > 20 and (want.mask()[solid != 0] & 0x3F == 0).sum() >= uncovered
+        a, b = got.loads(), want.loads()
+        assert (a.link_count, a.covered_count, a.uncovered_count) == (b.link_count, b.covered_count, b.uncovered_count)
+        assert np.array_equal(got.mask(), want.mask())
+        assert list(a.force) == list(b.force) and list(a.torque) == list(b.torque)
+        assert np.array_equal(got.populations(), want.populations())
+    # the whole box for one step only: then the bounds are the poses' again
+    again = build(0.4)
+    again.advance(20)
+    links = again.loads().link_count
+    again.restore_state(again.save_state())
+    again.advance(2)
+    assert abs(again.loads().link_count - links) < links
+
+
 def test_corrupted_checkpoint_fails_cleanly():
     cfg, _, _, _ = cases.shear_wave(n=16, viscosity=0.03, magic=3.0 / 16.0, axis="y")
     lat = lattice(cfg)
