@@ -1361,6 +1361,8 @@ __global__ void __launch_bounds__(128) k_topology(const GeomArgs a, int rep_s) {
 constexpr int kScanThreads = 256;
 constexpr int kScanPerThread = kScanSegment / kScanThreads;
 constexpr int kScanDirect = 2;
+// (links of a block of 256 cells: at most 18 a cell)
+static_assert((uint64_t)kScanDirect * kScanSegment * 256 * 18 <= 0xFFFFFFFFull, "these segments' links count in 32 bits");
 __device__ __forceinline__ uint32_t block_sum_scan(uint32_t v, uint32_t* wtot) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -1437,9 +1439,15 @@ __global__ void __maxnreg__(56) k_scan_apply(const GeomArgs a, int nseg) {
     for (int w = 0; w < warp; ++w) base += wtot[w];
     base += incl - mine;
     if ((int)blockIdx.x == nseg - 1 && threadIdx.x == kScanThreads - 1) {
-        const uint32_t total = base + mine;
+        // the list's offsets are 32 bits wide, its total is not: a list that wraps
+        // must raise the overflow flag
+        uint64_t total = base + mine;
+        if (nseg > kScanDirect) {
+            total = 0;
+            for (int k = 0; k < nseg; ++k) total += sums[k];
+        }
         if (ev) {
-            *a.b.event_total = total;  // at most one event a box cell
+            *a.b.event_total = (uint32_t)total;  // at most one event a box cell
         } else {
             a.b.state->link_count = (int64_t)total;
             a.b.state->link_overflow = total > a.b.link_capacity ? 1u : 0u;
