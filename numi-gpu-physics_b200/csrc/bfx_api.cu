@@ -19,6 +19,7 @@
 #include "bfx_clearance.h"
 #include "bfx_internal.h"
 #include "bfx_observation.h"
+#include "bfx_raster_order.h"
 #include "bfx_work_pool.h"
 
 using namespace bfx;
@@ -872,53 +873,6 @@ float geometry_radius(const bfx_config* c, const bfx_bird* b, const bfx_mesh* m)
     return r + c->mesh_half_thickness + 2.0f * c->cell_size;
 }
 
-// The triangles (vertices, id) in the order the raster takes them: along a Morton curve of the
-// centroid within each segment (10 bits an axis of the segment-frame
-// coordinates, the first keyframe's for a replay), every eighth triangle of the
-// curve first.  Those leave a key near the final one in almost every voxel,
-// which lets the others drop most of theirs; the order changes no result.
-std::vector<uint4> raster_order(const bfx_mesh* m) {
-    const float* pts = m->keyframe_count >= 2 ? m->keyframe_points : m->local_vertices;
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (uint32_t i = 0; i < m->vertex_count; ++i)
-        for (int k = 0; k < 3; ++k) {
-            lo[k] = std::min(lo[k], pts[3 * i + k]);
-            hi[k] = std::max(hi[k], pts[3 * i + k]);
-        }
-    // one scale for the three axes, so that the curve's cells are cubes
-    const float extent = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
-    const float scale = extent > 0.0f ? 1023.0f / (3.0f * extent) : 0.0f;
-    auto spread = [](uint32_t v) {
-        uint64_t r = 0;
-        for (int b = 0; b < 10; ++b) r |= (uint64_t)((v >> b) & 1u) << (3 * b);
-        return r;
-    };
-    std::vector<std::pair<uint64_t, uint32_t>> keyed(m->triangle_count);
-    for (uint32_t t = 0; t < m->triangle_count; ++t) {
-        const uint32_t* v = m->triangles + 3 * t;
-        uint64_t code = (uint64_t)m->vertex_segment[v[0]] << 32;
-        for (int k = 0; k < 3; ++k) {
-            const float c = (pts[3 * v[0] + k] - lo[k]) + (pts[3 * v[1] + k] - lo[k]) + (pts[3 * v[2] + k] - lo[k]);
-            const float f = c * scale;
-            const uint32_t i = f >= 0.0f ? (uint32_t)std::min(f, 1023.0f) : 0u;  // a NaN counts as 0
-            code |= spread(i) << k;
-        }
-        keyed[t] = {code, t};
-    }
-    std::sort(keyed.begin(), keyed.end());
-    std::vector<uint4> order;
-    order.reserve(m->triangle_count);
-    auto append = [&](uint32_t i) {
-        const uint32_t t = keyed[i].second;
-        const uint32_t* v = m->triangles + 3 * (size_t)t;
-        order.push_back(make_uint4(v[0], v[1], v[2], t));
-    };
-    for (uint32_t i = 0; i < m->triangle_count; i += 8) append(i);
-    for (uint32_t i = 0; i < m->triangle_count; ++i)
-        if (i % 8 != 0) append(i);
-    return order;
-}
-
 }  // namespace
 
 extern "C" {
@@ -1199,9 +1153,14 @@ int bfx_create(const bfx_config* config, const bfx_bird* bird, const bfx_body_st
             cudaMemcpyAsync(s->mesh_tris, mesh->triangles, (size_t)s->ntris * 3 * sizeof(uint32_t),
                             cudaMemcpyHostToDevice, s->stream);
             cudaMemcpyAsync(s->mesh_tri_part, mesh->triangle_part, s->ntris, cudaMemcpyHostToDevice, s->stream);
-            const std::vector<uint4> order = raster_order(mesh);
+            RasterOrder order;
+            if (!order.build(mesh)) {
+                bfx_destroy(s);
+                return fail(nullptr, BFX_ERR_ALLOCATION, "host memory for the triangle order");
+            }
+            static_assert(sizeof(RasterOrder::Triangle) == sizeof(uint4), "the device reads the records as uint4");
             BFX_ALLOC(s->mesh_order, (size_t)s->ntris * sizeof(uint4));
-            cudaMemcpyAsync(s->mesh_order, order.data(), (size_t)s->ntris * sizeof(uint4), cudaMemcpyHostToDevice,
+            cudaMemcpyAsync(s->mesh_order, order.triangles(), (size_t)s->ntris * sizeof(uint4), cudaMemcpyHostToDevice,
                             s->stream);
             if (mesh->keyframe_count >= 2) {
                 s->kf_count = (int)mesh->keyframe_count;
