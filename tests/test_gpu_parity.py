@@ -467,6 +467,91 @@ def test_lattice_faces_match_oracle(faces, extent, geometry):
     assert np.max(np.abs(wide.populations() - lat.populations())) < 100 * 2.0 ** -25
 
 
+def face_case(faces, extent, geometry=False, **kw):
+    """An extent with its own velocity on every face, an ellipsoid in its middle if asked for, and
+    populations 3 % around equilibrium."""
+    nx, ny, nz = extent
+    cfg, rows, body, _ = cases.ellipsoid_channel(nx=nx, ny=ny, nz=nz, radii=(1.2, 1.1, 1.4),
+                                                 center=(0.5 * nx, 0.5 * ny, 0.5 * nz), viscosity=0.03, **kw)
+    if not geometry:
+        cfg.geometry, rows, body = L.GEOMETRY_NONE, None, None
+    cfg.face_bc[:] = faces
+    for f in range(6):
+        cfg.face_velocity[f][:] = [0.04 - 0.01 * f, 0.01 * f, 0.005 * (f - 2)]
+    w = O.lattice()[2].astype(np.float64)[:, None, None, None]
+    start = (w * np.random.default_rng(5).uniform(0.97, 1.03, (19, nz, ny, nx))).astype(np.float32)
+    return cfg, rows, body, start
+
+
+@pytest.mark.parametrize("collision", [L.COLLISION_TRT_LIMITER, L.COLLISION_REGULARIZED, L.COLLISION_RR3])
+@pytest.mark.parametrize("faces", [[PE] * 6, [VE, FF, VE, VE, FF, VE], [VE, FF, PE, PE, FF, VE]])
+@pytest.mark.parametrize("geometry", [False, True])
+def test_lattice_faces_of_every_operator_match_oracle(collision, faces, geometry):
+    """The faces inside the kernel for the other operators, the last step capturing fields."""
+    cfg, rows, body, start = face_case(faces, (35, 9, 11), geometry, collision=collision)
+    lat, osim = make_pair(cfg, rows, body)
+    lat.set_populations(start)
+    osim.pa[:] = start.ravel()
+    for step in range(4):
+        lat.advance(1, capture_fields=step == 3)
+        osim.step()
+        assert compare_pops(lat, osim, f"step {step + 1}")[1]
+    density, velocity = lat.fields()
+    c = O.lattice()[0].astype(np.float64)
+    pops = lat.populations().reshape(19, -1).astype(np.float64)
+    fluid = np.ones(pops.shape[1], bool) if not geometry else (lat.mask() & 0x3F) == 0
+    # 19 FP32 additions with partial sums up to about 1
+    assert np.max(np.abs(density - pops.sum(0))[fluid]) < 40 * 2.0 ** -24
+    u = (pops.T @ c) / pops.sum(0)[:, None]
+    assert np.max(np.abs(velocity - u)[fluid]) < 40 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("collision", [L.COLLISION_TRT, L.COLLISION_REGULARIZED, L.COLLISION_RR3, L.COLLISION_TRT_LIMITER])
+@pytest.mark.parametrize("storage", [L.STORAGE_F16_DEVIATION, L.STORAGE_BF16_DEVIATION])
+@pytest.mark.parametrize("faces", [[VE, FF, VE, VE, FF, VE], [VE] * 6, [VE, FF, PE, PE, VE, VE], [PE, PE, VE, FF, VE, FF],
+                                   [VE, OU, VE, FF, PE, PE]])
+@pytest.mark.parametrize("extent", [(65, 9, 8), (33, 17, 5), (5, 4, 31), (130, 16, 4)])
+def test_16bit_lattice_faces_stay_within_their_quantum_of_fp64(collision, storage, faces, extent):
+    """Every face, edge and corner of the half-storage step, with and without a fill: each step against
+    the FP64 one from the same populations.  The inputs are equal but for the face values, stored to q
+    of their deviation; the output is stored to q of its own (a stochastic store to twice that), and
+    the collision's gain is below 2: 4 q of the larger deviation, and FP32 rounding."""
+    cfg, _, _, start = face_case(faces, extent, storage=storage, collision=collision)
+    half = Lattice(cfg)
+    cfg.storage = L.STORAGE_F64
+    wide = Lattice(cfg)
+    _, _, w = O.lattice()
+    w = w.astype(np.float64)[:, None]
+    q = 2.0 ** -11 if storage == L.STORAGE_F16_DEVIATION else 2.0 ** -8
+    half.set_populations(start)
+    # the largest deviation a face value has: w_q (3 c.u + ...) of the rest and axis directions
+    face_deviation = 1.0 / 18.0 * (3 * 0.055 + 9 * 0.055 ** 2)
+    for _ in range(4):
+        wide.set_populations(half.populations())
+        half.advance(1)
+        wide.advance(1)
+        a, b = (lat.populations().reshape(19, -1).astype(np.float64) for lat in (half, wide))
+        d = np.maximum(np.abs(b - w).max(axis=0), face_deviation)[None, :]
+        assert np.max(np.abs(a - b) / (4.0 * q * d + 4e-7 * w)) <= 1.0
+
+
+@pytest.mark.parametrize("center", [(6.61, 9.3, 8.8), (17.39, 9.3, 8.8), (12.1, 6.61, 8.8), (12.1, 9.3, 11.39),
+                                    (6.59, 6.62, 6.6), (5.5, 9.3, 8.8), (20.5, 9.3, 8.8)])
+def test_static_body_at_the_limit_of_the_side_fill_matches_oracle(center):
+    """A static body whose solid cells begin three cells from a face (the fill then runs beside the
+    links), two and fewer, beside velocity, outflow and periodic faces.  (Not across a periodic face:
+    the oracle, as the reference, has no link fraction there.)"""
+    cfg, rows, body, _ = cases.ellipsoid_channel(nx=24, ny=18, nz=18, radii=(3.6, 3.6, 3.6), center=center,
+                                                 viscosity=0.02, collision=L.COLLISION_TRT)
+    lat, osim = make_pair(cfg, rows, body)
+    for _ in range(8):
+        lat.advance(5, batch_size=5)
+        for _ in range(5):
+            osim.step()
+        assert compare_pops(lat, osim, f"center {center}")[1]
+        assert np.array_equal(lat.mask(), osim.mcur)
+
+
 # --------------------------------------------------------------------------
 # Mesh raster: order and size of the triangles
 # --------------------------------------------------------------------------
