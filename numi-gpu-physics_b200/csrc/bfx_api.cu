@@ -368,6 +368,25 @@ void encode_geometry_build(bfx_sim* s, int init, uint8_t* mprev, uint8_t* mnext)
 // is done by the link kernel before the fluid kernel, and the box's solid
 // cells (which read the wall field) are launched before the fork.
 bool can_pipeline(const bfx_sim* s) { return s->moving() && s->side != nullptr; }
+// ... and whether `count` steps in a batch gain by it.  The batch's first step
+// and its last one or two are launched directly, which takes some 20-60 us of
+// host time more than graph replays where the GPU does not hide it; a step gains
+// about half of what the fluid kernel takes beyond 9 us (below that the forks and
+// joins cost what the overlap saves).  Measured per step, graphs -> pipelined: plates FP32 64 x 40 x 40
+// batches of 3 77 -> 104 us, of 32 72 -> 78; 128 x 72 x 72 of 4 99 -> 107, of 16
+// 95 -> 93; 256 x 136 x 136 of 2 291 -> 263, of 32 276 -> 221; FP64 128 x 72 x 72 of
+// 4 137 -> 130; coupled bird 64^3 of 12 57 -> 60.  The staged kernel's steps are
+// pipelined from two on: what follows it alone takes as long as it.
+bool pipeline_pays(const bfx_sim* s, uint64_t count) {
+    if (!can_pipeline(s) || count < 2) return false;
+    if (s->tma_ok) return true;
+    // fluid kernel, us per million cells
+    const bool limiter = s->cfg.collision == BFX_COLLISION_TRT_LIMITER;
+    const double rate = s->cfg.storage == BFX_STORAGE_F64   ? (limiter ? 139.0 : 65.0)
+                        : s->cfg.storage == BFX_STORAGE_F32 ? (limiter ? 60.0 : 32.0)
+                                                            : 40.0;
+    return 0.55 * (1.0e-6 * (double)s->g.n * rate - 9.0) * (double)(count - 1) > 35.0;
+}
 
 // Faces f0..f1 are far-field or velocity faces: the values the halo fill
 // writes there depend only on the face and the direction.
@@ -711,13 +730,13 @@ int run_graphs(bfx_sim* s, uint64_t& k, uint64_t limit, bool pipelined = false) 
     return BFX_OK;
 }
 
-// `count` steps without capture, samples or tape.  Pipelined where possible:
+// `count` steps without capture, samples or tape.  Pipelined where that pays:
 // every step but the last builds the next step's geometry beside its own fluid
 // kernel; the first builds its own, pairs replay a graph while a step remains
 // after them, the last one or two run directly.
 int run_plain_steps(bfx_sim* s, uint64_t count) {
     uint64_t k = 0;
-    if (s->graphs_enabled && !s->timing && !s->topo_mode && can_pipeline(s) && count > 1) {
+    if (s->graphs_enabled && !s->timing && !s->topo_mode && pipeline_pays(s, count)) {
         encode_step(s, 0, nullptr, 0, nullptr, nullptr, false, true);
         k = 1;
         const int rc = run_graphs(s, k, count - 1, true);
@@ -1347,7 +1366,7 @@ int bfx_advance(bfx_sim* s, uint64_t steps, uint32_t batch_size, uint32_t flags,
         // Pairs of plain steps replay a captured graph; steps that capture
         // fields, record samples or are individually timed are encoded directly.
         const bool last_batch = done + count == steps;
-        if (s->graphs_enabled && !record && !s->timing && !s->topo_mode && can_pipeline(s) && count > 1) {
+        if (s->graphs_enabled && !record && !s->timing && !s->topo_mode && pipeline_pays(s, count)) {
             // Pipelined: every step but the batch's last builds the next
             // step's geometry beside its own fluid kernel.  The batch's first
             // step builds its own; pairs replay a graph while a step of the

@@ -97,6 +97,31 @@ def test_every_step_without_geometry_is_counted_once(storage, collision, faces, 
     assert lat.step_index()[0] == 85
 
 
+@pytest.mark.parametrize("name", ["plates", "plates fast_math", "bird", "wing"])
+def test_large_single_precision_batches_equal_single_steps(name):
+    """Lattices whose FP32 steps are pipelined (the small ones above replay graphs), in batches on both
+    sides of the rule, against one-step calls: bit for bit."""
+    def build():
+        if name == "bird":
+            from bfx.simulation import BirdFlowSimulation
+            return BirdFlowSimulation(*cases.compact_bird(free_flight=True, n=128)).lattice
+        if name == "wing":
+            cfg, wing = cases.flapping_wing(chord=12, cycle_steps=480, viscosity=0.02)
+            return Lattice(cfg, wing=wing)
+        cfg, rows, body, mesh = small_mesh_case(nx=192, ny=104, nz=104)
+        cfg.fast_math = int("fast" in name)
+        return lattice(cfg, rows, body, mesh)
+    batched, single = build(), build()
+    for batch in (20, 2, 3, 11, 4):
+        batched.advance(batch, batch_size=batch)
+    for _ in range(40):
+        single.advance(1, batch_size=1)
+    assert batched.step_index()[0] == single.step_index()[0] == 40
+    assert np.array_equal(batched.populations(), single.populations())
+    a, b = batched.loads(), single.loads()
+    assert list(a.force) == list(b.force) and list(a.torque) == list(b.torque) and a.link_count == b.link_count
+
+
 @pytest.mark.parametrize("extent,storage,collision,launches", [
     ((64, 64, 64), L.STORAGE_F32, L.COLLISION_TRT, 1), ((4096, 16, 16), L.STORAGE_F32, L.COLLISION_RR3, 1),
     ((8, 400, 400), L.STORAGE_F32, L.COLLISION_TRT, 2), ((33, 150, 150), L.STORAGE_F32, L.COLLISION_TRT_LIMITER, 2),
