@@ -906,7 +906,8 @@ static void adjoint_step_t(int rep_s, const GridDesc& gd, const BoxDesc& box, Ad
     const int64_t halo = a.ga.g.pn - a.ga.g.n;
     k_adj_halo<R><<<(unsigned)((halo + 127) / 128), 128, 0, s>>>(a, rep_s, halo);
     k_adj_topology<R><<<bgrid, bblock, 0, s>>>(a, rep_s);
-    k_adj_reduce<<<1, kAdjReduceThreads, 0, s>>>(a.part_rare, (int)(bgrid.x * bgrid.y * bgrid.z), a.part_links, apply_blocks, a.obj);
+    k_adj_reduce<<<1, kAdjReduceThreads, 0, s>>>(a.part_rare, (int)(bgrid.x * bgrid.y * bgrid.z), a.part_links,
+                                                 apply_blocks, a.obj);
 }
 
 static AdjArgs adjoint_args(int storage, const GridDesc& g, const FluidParams& fp, const BoxDesc& box,

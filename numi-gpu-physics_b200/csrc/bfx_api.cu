@@ -241,7 +241,9 @@ size_t work_limit() {
 }
 
 // Device memory for the handle.
-cudaError_t handle_malloc(bfx_sim* s, void** p, size_t bytes) { return (cudaError_t)g_work.allocate(s->device, p, bytes); }
+cudaError_t handle_malloc(bfx_sim* s, void** p, size_t bytes) {
+    return (cudaError_t)g_work.allocate(s->device, p, bytes);
+}
 
 template <class T>
 cudaError_t dalloc(bfx_sim* s, T** p, size_t bytes) {
@@ -633,7 +635,8 @@ void encode_step(bfx_sim* s, int capture, bfx_run_sample* sample_slot_base, uint
                     s->geometry() ? box : nullptr, s->stream);
         timing_end(s);
     }
-    s->launches += pipelined ? 2 : launch_bulk_count(s->cfg.storage, s->cfg.collision, capture, s->tma_ok, s->geometry());
+    s->launches +=
+        pipelined ? 2 : launch_bulk_count(s->cfg.storage, s->cfg.collision, capture, s->tma_ok, s->geometry());
     GeomBuffers gb = geom_buffers(s, mprev, mnext);
     if (!finish_fused && !counted && !tape) {
         launch_integrate(s->g, s->fp, gb, fin.gravity[0], fin.gravity[1], fin.gravity[2], fin.substeps,
@@ -674,10 +677,10 @@ void drop_graphs(bfx_sim* s) {
         }
 }
 
-// Replays (capturing on first use) the graph of `nsteps` (1, 2 or kLongSteps) plain steps
-// for the current parity.  Host-side state (representation, mask index)
-// alternates with period two, so a pair graph leaves it where it started and
-// the single-step graph of each parity hands over to the other's.  A pipelined
+// Replays (capturing on first use) the graph of `nsteps` (1, 2 or kLongSteps)
+// plain steps for the current parity.  Host-side state (representation, mask
+// index) alternates with period two, so a pair graph leaves it where it started
+// and the single-step graph of each parity hands over to the other's.  A pipelined
 // pair takes its first step's geometry as built and builds the geometry of the
 // step after the pair (so one more step of the same batch must follow).
 int run_steps_graph(bfx_sim* s, int nsteps, bool pipelined = false) {

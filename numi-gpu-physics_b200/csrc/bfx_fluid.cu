@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(128) k_halo(const BulkArgs a, int rep_s, int64
 // the face and the direction.  When both x faces (or all six) are of those
 // kinds the staged kernel takes their values from this table and their halo
 // fill is skipped (an x face's is one scattered store per row and direction):
-// out[19 f + q] = the stored value of direction q across face f, read back as the staged kernel reads a population (scaled deviation).
+// out[19 f + q] = the stored value of direction q across face f, read back as
+// the staged kernel reads a population (scaled deviation).
 template <class S>
 __global__ void k_halo_values(const BulkArgs a, float* out) {
     using T = typename S::T;

@@ -217,9 +217,9 @@ __device__ __forceinline__ uint32_t link_sources(const Grid& g, const uint8_t* m
 }
 
 __device__ __forceinline__ float tri_distance(const GeomArgs& a, uint32_t t, V3 w) {
-    V3 A, B, C;
+    V3 A, B, C, bary;
     tri_vertices(a, t, A, B, C);
-    return closest_distance(w, A, B, C);
+    return length(w - closest_point(w, A, B, C, bary));
 }
 
 __device__ __forceinline__ unsigned long long box_key(const GeomArgs& a, int x, int y, int z) {

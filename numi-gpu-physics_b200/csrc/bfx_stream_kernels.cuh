@@ -465,7 +465,8 @@ __global__ void __maxnreg__(StreamShape<COLL>::max_regs)
                 float r = __fmaf_rn(fp.far[3] - r0, s, r0);
                 r = r > 1.0e-8f ? r : 1.0e-8f;
                 const float inv = 1.0f / r;
-                const float mx = Lanes<P2>::get(ux, l) * r0, my = Lanes<P2>::get(uy, l) * r0, mz = Lanes<P2>::get(uz, l) * r0;
+                const float mx = Lanes<P2>::get(ux, l) * r0, my = Lanes<P2>::get(uy, l) * r0,
+                            mz = Lanes<P2>::get(uz, l) * r0;
                 const uint32_t gl = gida + 32 * l;
                 a.density[gl] = r;
                 a.velocity[gl] = make_float4(__fmaf_rn(fp.far[3] * fp.far[0] - mx, s, mx) * inv,

@@ -92,7 +92,8 @@ BFX_HD float closest_distance(V3 p, V3 a, V3 b, V3 c) {
     const float num = r == 2 ? d1 : (r == 4 ? d2 : (r == 5 ? d4 - d3 : 1.0f));
     const float den = r == 2 ? d1 - d3
                              : (r == 4 ? d2 - d6
-                                       : (r == 5 ? (d4 - d3) + (d5 - d6) : (r == 6 ? fmaxf(va + vb + vc, 1.0e-20f) : 1.0f)));
+                                       : (r == 5 ? (d4 - d3) + (d5 - d6)
+                                                 : (r == 6 ? fmaxf(va + vb + vc, 1.0e-20f) : 1.0f)));
     const float quot = num / den;
     const float s = r == 6 ? vb * quot : (r == 2 || r == 4 || r == 5 ? quot : 0.0f);
     const float t = r == 6 ? vc * quot : 0.0f;

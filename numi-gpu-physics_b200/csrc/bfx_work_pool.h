@@ -85,7 +85,8 @@ class WorkPool {
                 }
                 kept += blocks[i].bytes;
                 int old;
-                while ((old = oldest(device)) >= 0 && bytes_on(device) > limit - blocks[i].bytes) freed[nfreed++] = remove(old);
+                while ((old = oldest(device)) >= 0 && bytes_on(device) > limit - blocks[i].bytes)
+                    freed[nfreed++] = remove(old);
                 if (count_ == kMaxBlocks) freed[nfreed++] = remove(0);
                 kept_[count_++] = Block{blocks[i].p, blocks[i].bytes, device, owner};
             }

@@ -506,10 +506,11 @@ def test_lattice_faces_of_every_operator_match_oracle(collision, faces, geometry
     assert np.max(np.abs(velocity - u)[fluid]) < 40 * 2.0 ** -24
 
 
-@pytest.mark.parametrize("collision", [L.COLLISION_TRT, L.COLLISION_REGULARIZED, L.COLLISION_RR3, L.COLLISION_TRT_LIMITER])
+@pytest.mark.parametrize("collision", [L.COLLISION_TRT, L.COLLISION_REGULARIZED, L.COLLISION_RR3,
+                                       L.COLLISION_TRT_LIMITER])
 @pytest.mark.parametrize("storage", [L.STORAGE_F16_DEVIATION, L.STORAGE_BF16_DEVIATION])
-@pytest.mark.parametrize("faces", [[VE, FF, VE, VE, FF, VE], [VE] * 6, [VE, FF, PE, PE, VE, VE], [PE, PE, VE, FF, VE, FF],
-                                   [VE, OU, VE, FF, PE, PE]])
+@pytest.mark.parametrize("faces", [[VE, FF, VE, VE, FF, VE], [VE] * 6, [VE, FF, PE, PE, VE, VE],
+                                   [PE, PE, VE, FF, VE, FF], [VE, OU, VE, FF, PE, PE]])
 @pytest.mark.parametrize("extent", [(65, 9, 8), (33, 17, 5), (5, 4, 31), (130, 16, 4)])
 def test_16bit_lattice_faces_stay_within_their_quantum_of_fp64(collision, storage, faces, extent):
     """Every face, edge and corner of the half-storage step, with and without a fill: each step against
