@@ -269,7 +269,7 @@ __device__ DV closest_point_dual(V3 p, const DV& a, const DV& b, const DV& c, Du
         return b;
     }
     const Du vc = d1 * d4 - d3 * d2;
-    if (vc.v <= 0.0f && d1.v >= 0.0f && d3.v <= 0.0f && d1.v > d3.v) {
+    if (vc.v <= 0.0f && d1.v >= 0.0f && d3.v < 0.0f) {
         const Du v = d1 / (d1 - d3);
         bary[0] = dc(1.0f) - v;
         bary[1] = v;
@@ -285,7 +285,7 @@ __device__ DV closest_point_dual(V3 p, const DV& a, const DV& b, const DV& c, Du
         return c;
     }
     const Du vb = d5 * d2 - d1 * d6;
-    if (vb.v <= 0.0f && d2.v >= 0.0f && d6.v <= 0.0f && d2.v > d6.v) {
+    if (vb.v <= 0.0f && d2.v >= 0.0f && d6.v < 0.0f) {
         const Du w = d2 / (d2 - d6);
         bary[0] = dc(1.0f) - w;
         bary[1] = dc(0.0f);

@@ -789,9 +789,10 @@ __global__ void k_mesh_clear(const GeomArgs a) {
 // what is left is queued, so that the distance search runs on full warps,
 // without branches (closest_distance).  Keys are minima, so the order of the
 // atomics changes no result.
-// 145 k triangles (768 x 384 x 384 bird) 407 -> 278 us against one warp per
-// triangle over every voxel of its box; 16 k triangles 50 -> 52 us: there the
-// whole mesh is in flight at once and finds no keys to drop by.
+// Alone and cold, against one warp per triangle over every voxel of its box:
+// 145 k triangles (768 x 384 x 384 bird) 407 -> 289 us, 16 k (512 x 256 x 256
+// plates) 50 -> 41, where the whole mesh is in flight at once and finds few keys
+// to drop by.
 constexpr int kRasterTris = 4;
 struct RasterTri {
     float cen[3], reach2;

@@ -25,8 +25,11 @@ BFX_HD float length(V3 a) { return sqrtf(dot(a, a)); }
 
 // Closest point of triangle (a, b, c) to p and its barycentric coordinates.  An
 // edge region needs an edge: where its two end distances are equal (an edge of
-// zero length, or one that rounds to it) the region's quotient would be 0 / 0, and
-// the following regions hold the point: with a = b the edge region a-c.
+// zero length, or one that rounds to it) its quotient would be 0 / 0, and the
+// following regions hold the point: with a = b the edge region a-c.  Hence d3 < 0
+// and d6 < 0 where the reference has <=: with d3 = 0 the region's other
+// conditions leave d1 = 0 alone, as d1 d4 <= 0 and, past b's region, d4 > 0
+// (likewise d6 = 0 and d2).
 BFX_HD V3 closest_point(V3 p, V3 a, V3 b, V3 c, V3& bary) {
     V3 ab = b - a, ac = c - a, ap = p - a;
     float d1 = dot(ab, ap), d2 = dot(ac, ap);
@@ -41,7 +44,7 @@ BFX_HD V3 closest_point(V3 p, V3 a, V3 b, V3 c, V3& bary) {
         return b;
     }
     float vc = d1 * d4 - d3 * d2;
-    if (vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f && d1 > d3) {
+    if (vc <= 0.0f && d1 >= 0.0f && d3 < 0.0f) {
         float v = d1 / (d1 - d3);
         bary = v3(1.0f - v, v, 0);
         return v3(a.x + v * ab.x, a.y + v * ab.y, a.z + v * ab.z);
@@ -53,7 +56,7 @@ BFX_HD V3 closest_point(V3 p, V3 a, V3 b, V3 c, V3& bary) {
         return c;
     }
     float vb = d5 * d2 - d1 * d6;
-    if (vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f && d2 > d6) {
+    if (vb <= 0.0f && d2 >= 0.0f && d6 < 0.0f) {
         float w = d2 / (d2 - d6);
         bary = v3(1.0f - w, 0, w);
         return v3(a.x + w * ac.x, a.y + w * ac.y, a.z + w * ac.z);
@@ -82,9 +85,9 @@ BFX_HD float closest_distance(V3 p, V3 a, V3 b, V3 c) {
     const float vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
     const bool in_a = d1 <= 0.0f && d2 <= 0.0f;
     const bool in_b = d3 >= 0.0f && d4 <= d3;
-    const bool on_ab = vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f && d1 > d3;
+    const bool on_ab = vc <= 0.0f && d1 >= 0.0f && d3 < 0.0f;
     const bool in_c = d6 >= 0.0f && d5 <= d6;
-    const bool on_ac = vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f && d2 > d6;
+    const bool on_ac = vb <= 0.0f && d2 >= 0.0f && d6 < 0.0f;
     const bool on_bc =
         va <= 0.0f && (d4 - d3) >= 0.0f && (d5 - d6) >= 0.0f && (d4 - d3) + (d5 - d6) > 0.0f;
     // 0 a, 1 b, 2 ab, 3 c, 4 ac, 5 bc, 6 face

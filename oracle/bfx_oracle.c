@@ -1492,7 +1492,7 @@ static void closest_point(const float p[3], const float a[3], const float b[3], 
         return;
     }
     float vc = d1 * d4 - d3 * d2;
-    if (vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f && d1 > d3) {
+    if (vc <= 0.0f && d1 >= 0.0f && d3 < 0.0f) {
         float v = d1 / (d1 - d3);
         for (int k = 0; k < 3; ++k) out[k] = a[k] + v * ab[k];
         bary[0] = 1.0f - v; bary[1] = v; bary[2] = 0;
@@ -1506,7 +1506,7 @@ static void closest_point(const float p[3], const float a[3], const float b[3], 
         return;
     }
     float vb = d5 * d2 - d1 * d6;
-    if (vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f && d2 > d6) {
+    if (vb <= 0.0f && d2 >= 0.0f && d6 < 0.0f) {
         float w = d2 / (d2 - d6);
         for (int k = 0; k < 3; ++k) out[k] = a[k] + w * ac[k];
         bary[0] = 1.0f - w; bary[1] = 0; bary[2] = w;
