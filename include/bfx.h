@@ -468,7 +468,7 @@ BFX_API int bfx_launch_count(bfx_sim* sim, uint64_t* launches);
 BFX_API int bfx_device_bytes(bfx_sim* sim, uint64_t* bytes);
 /* Frees the device memory that gradients (bfx_adjoint) on this handle's device
  * left for the next ones: at most 8 GiB a device and a quarter of what was free
- * when a gradient returned.  The library gives it back by itself before an
+ * when the gradient that allocated it returned.  The library gives it back by itself before an
  * allocation of any handle fails, and with the handle whose gradient left it;
  * this call is for other allocators of the process. */
 BFX_API int bfx_release_work_memory(bfx_sim* sim);

@@ -174,6 +174,7 @@ class WorkCall {
             const int status = pool_.allocate(device_, &b.p, n);
             if (status != 0) return status;
             b.bytes = n;
+            allocated_ = true;
         }
         used_[count_++] = b;
         *p = (T*)b.p;
@@ -186,6 +187,8 @@ class WorkCall {
         count_ = 0;
     }
     uint64_t bytes() const { return bytes_; }
+    // Some of the blocks are new, not from the list.
+    bool allocated() const { return allocated_; }
 
   private:
     WorkPool& pool_;
@@ -194,6 +197,7 @@ class WorkCall {
     WorkPool::Block used_[WorkPool::kMaxBlocks] = {};
     int count_ = 0;
     uint64_t bytes_ = 0;
+    bool allocated_ = false;
 };
 
 }  // namespace bfx

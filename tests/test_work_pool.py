@@ -57,11 +57,11 @@ static int a_call_finds_the_blocks_of_the_last() {
     { WorkCall c(pool, 0, &A); CHECK(c.get(&p, 1000000) == 0 && c.get(&q, 0) == 0 && c.bytes() == 1000016);
       first[0] = p; first[1] = q; c.keep(1 << 30); }
     CHECK(used == 1000016 && pool.held(&A) == 1000016 && pool.held(&B) == 0);
-    { WorkCall c(pool, 0, &B); CHECK(c.get(&p, 900000) == 0 && p == first[0] && allocations == 2);
+    { WorkCall c(pool, 0, &B); CHECK(c.get(&p, 900000) == 0 && p == first[0] && allocations == 2 && !c.allocated());
       CHECK(pool.held(&A) == 16); c.keep(1 << 30); }
     CHECK(pool.held(&B) == 1000000 && pool.held(&A) == 16);
     { WorkCall c(pool, 0, &A); CHECK(c.get(&p, 700000) == 0 && p != first[0]);    // a quarter wasted: not taken
-      void* r = nullptr; CHECK(c.get(&r, 1000001) == 0 && r != first[0]); c.keep(1 << 30); }
+      void* r = nullptr; CHECK(c.get(&r, 1000001) == 0 && r != first[0] && c.allocated()); c.keep(1 << 30); }
     CHECK(pool.held(&A) == 1700001);                  // its 16 bytes, not used again, were freed
     WorkCall other(pool, 1, &A);                      // another device's blocks are no use
     CHECK(other.get(&p, 1000000) == 0 && p != first[0] && pool.held(&B) == 1000000);
